@@ -7,9 +7,9 @@
 
 namespace ppml_b200 {
 
-// Strided batched contraction on CUDA cores (simt_kernels.cu).
+// Strided batched contraction on CUDA cores (simt_contract.cu).
 //   D[plane][m][n] = epi( sum_k A[..][m*a_sm + k*a_sk] * B[..][n*b_sn + k*b_sk] )
-// plane = i3*ne2 + i2; A's plane is (i2 / a_div2, i3 / a_div3) (broadcast as the reference's CPU
+// plane = i3*ne2 + i2; A's plane is (i2 / a_div2, i3 / a_div3), B's likewise (broadcast as the reference's CPU
 // out_prod does, src/backend/CPUKernels.cpp:836-858).
 struct SimtContract {
     long long M, N, K;
@@ -18,6 +18,9 @@ struct SimtContract {
     long long planes, ne2;
     long long a_s2, a_s3, a_div2, a_div3;
     long long b_s2, b_s3, c_s2, c_s3;
+    long long b_div2, b_div3;   // 0 = 1
+    int may_split;              // 1: the contraction may be split over CTAs (changes the summation order)
+    int vec_c;                  // set by the launcher: 16-byte stores are legal
     const float* bias;
     int bias_seed;              // 1: accumulator starts at bias[n] (fp32 mul_mat); 0: added at the end
     float alpha;

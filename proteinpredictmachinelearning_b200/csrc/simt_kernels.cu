@@ -1,7 +1,5 @@
-// simt_kernels.cu -- CUDA-core kernels: exact-fp32 contraction for every shape the tensor-core
-// paths do not take (unaligned K, inner batch > 1, tiny extents), the block quantizers, casts, the
-// dp4a Q8 product and the general attention kernel.  They keep the reference's summation order
-// (k ascending per output element) so fp32 results agree with its CPU kernels to rounding.
+// simt_kernels.cu -- CUDA-core kernels: LayerNorm statistics, the block quantizers, casts, the dp4a Q8 product and
+// the general attention kernels.
 #include "kernels.h"
 
 #include <cuda_bf16.h>
@@ -24,119 +22,6 @@ int* device_error_ptr() {
         cached[dev] = p;
     }
     return cached[dev];
-}
-
-// =============================================================================================
-// Generic strided batched contraction:  D[p][m][n] = epi( sum_k A[pa][m][k] * B[pb][n][k] )
-// 64 x 64 output tile, 16-deep K slices, 256 threads, 4 x 4 outputs per thread.
-// =============================================================================================
-template <typename T> __device__ __forceinline__ float to_f32(T v);
-template <> __device__ __forceinline__ float to_f32<float>(float v) { return v; }
-template <> __device__ __forceinline__ float to_f32<__half>(__half v) { return __half2float(v); }
-template <> __device__ __forceinline__ float to_f32<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
-
-template <typename T, bool A_KFAST, bool B_KFAST>
-__global__ void __launch_bounds__(256)
-simt_contract_kernel(const T* __restrict__ A, const T* __restrict__ B, float* __restrict__ C, SimtContract p) {
-    __shared__ float As[16][64 + 4];
-    __shared__ float Bs[16][64 + 4];
-    const int tid = threadIdx.x;
-    const int tx = tid & 15, ty = tid >> 4;
-    const long long m0 = static_cast<long long>(blockIdx.y) * 64, n0 = static_cast<long long>(blockIdx.x) * 64;
-
-    for (long long plane = blockIdx.z; plane < p.planes; plane += gridDim.z) {
-        const long long i3 = plane / p.ne2, i2 = plane - i3 * p.ne2;
-        const T* Ap = A + (i2 / p.a_div2) * p.a_s2 + (i3 / p.a_div3) * p.a_s3;
-        const T* Bp = B + i2 * p.b_s2 + i3 * p.b_s3;
-        float* Cp = C + i2 * p.c_s2 + i3 * p.c_s3;
-
-        float acc[4][4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const long long n = n0 + tx * 4 + j;
-                acc[i][j] = (p.bias_seed && p.bias != nullptr && n < p.N) ? p.bias[n] : 0.0f;
-            }
-
-        for (long long k0 = 0; k0 < p.K; k0 += 16) {
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int idx = tid + i * 256;
-                int mm, kk;
-                if (A_KFAST) { kk = idx & 15; mm = idx >> 4; } else { mm = idx & 63; kk = idx >> 6; }
-                const long long m = m0 + mm, k = k0 + kk;
-                As[kk][mm] = (m < p.M && k < p.K) ? to_f32<T>(Ap[m * p.a_sm + k * p.a_sk]) : 0.0f;
-                int nn, kb;
-                if (B_KFAST) { kb = idx & 15; nn = idx >> 4; } else { nn = idx & 63; kb = idx >> 6; }
-                const long long n = n0 + nn, k2 = k0 + kb;
-                Bs[kb][nn] = (n < p.N && k2 < p.K) ? to_f32<T>(Bp[n * p.b_sn + k2 * p.b_sk]) : 0.0f;
-            }
-            __syncthreads();
-#pragma unroll
-            for (int kk = 0; kk < 16; ++kk) {
-                float a[4], b[4];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) a[i] = As[kk][ty * 4 + i];
-#pragma unroll
-                for (int j = 0; j < 4; ++j) b[j] = Bs[kk][tx * 4 + j];
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-            }
-            __syncthreads();
-        }
-
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const long long m = m0 + ty * 4 + i;
-            if (m >= p.M) continue;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const long long n = n0 + tx * 4 + j;
-                if (n >= p.N) continue;
-                float v = acc[i][j] * p.alpha;
-                if (p.ln_stats != nullptr) {           // LayerNorm folded into the Linear (bias_seed is 0 here)
-                    const float2 st2 = *reinterpret_cast<const float2*>(p.ln_stats + 2 * m);
-                    v = fmaf(-st2.x, p.ln_u[n], v) * st2.y;
-                }
-                if (!p.bias_seed && p.bias != nullptr) v += p.bias[n];
-                if (p.clamp) {
-                    if (!(v == v)) v = 0.0f; else v = fminf(fmaxf(v, -1e4f), 1e4f);
-                }
-                if (p.opm_L > 0) {
-                    const long long d1 = m / p.opm_L, ii = m - d1 * p.opm_L;
-                    const long long d2 = n / p.opm_L, jj = n - d2 * p.opm_L;
-                    Cp[(((d1 * p.opm_D + d2) * p.opm_L + ii) * p.opm_L + jj) * p.opm_B] = v;
-                } else {
-                    if (p.gate != nullptr) v = act_scalar(p.act, v) * p.gate[m * p.c_sm + n * p.c_sn];
-                    else if (p.act != 0) v = act_scalar(p.act, v);
-                    Cp[m * p.c_sm + n * p.c_sn] = v;
-                }
-            }
-        }
-    }
-}
-
-template <typename T>
-static int launch_contract_t(const T* A, const T* B, float* C, const SimtContract& p, cudaStream_t st) {
-    if (p.M <= 0 || p.N <= 0 || p.planes <= 0) return ST_BAD_ARGS;
-    dim3 grid(static_cast<unsigned>((p.N + 63) / 64), static_cast<unsigned>((p.M + 63) / 64),
-              static_cast<unsigned>(p.planes < 32768 ? p.planes : 32768));
-    if (grid.y > 65535u) return ST_BAD_ARGS;
-    const bool ak = (p.a_sk == 1), bk = (p.b_sk == 1);
-    if (ak && bk) simt_contract_kernel<T, true, true><<<grid, 256, 0, st>>>(A, B, C, p);
-    else if (ak) simt_contract_kernel<T, true, false><<<grid, 256, 0, st>>>(A, B, C, p);
-    else if (bk) simt_contract_kernel<T, false, true><<<grid, 256, 0, st>>>(A, B, C, p);
-    else simt_contract_kernel<T, false, false><<<grid, 256, 0, st>>>(A, B, C, p);
-    return cudaGetLastError() == cudaSuccess ? ST_OK : ST_LAUNCH;
-}
-
-int launch_simt_contract(const void* A, const void* B, float* C, const SimtContract& p, int elem, cudaStream_t st) {
-    if (elem == 0) return launch_contract_t<float>(static_cast<const float*>(A), static_cast<const float*>(B), C, p, st);
-    if (elem == 1) return launch_contract_t<__half>(static_cast<const __half*>(A), static_cast<const __half*>(B), C, p, st);
-    return launch_contract_t<__nv_bfloat16>(static_cast<const __nv_bfloat16*>(A), static_cast<const __nv_bfloat16*>(B), C, p, st);
 }
 
 // =============================================================================================

@@ -778,6 +778,27 @@ def test_out_prod(oracle):
             assert abs(got[i1, i0] - sum(float(a[i0 + k * 4]) * float(b[i1 + k * 5]) for k in range(3))) <= 1e-4
 
 
+@pytest.mark.parametrize("M,K,N", [(64, 16, 64), (65, 15, 127), (129, 17, 33), (127, 20, 32), (28480, 20, 132), (28481, 4, 128), (130, 36, 1)])
+def test_exact_contraction_tile_edges(oracle, M, K, N):
+    """Edges of the exact contraction's tiles (64 x 64, 64 x 128 from 444 tiles on, 128 x 32) and of its slices of 16, with
+    vector and element-wise loads and stores."""
+    a, b, bi = cases.mul_mat_case(M, K, N, seed=31)
+    got = host(ops.mul_mat_cuda(dev(a), dev(b), dev(bi), path=PATH_SIMT))
+    rows = np.unique(np.r_[0:min(M, 200), max(0, M - 200):M])
+    assert cases.rel_err(got[rows], oracle.mul_mat_f32(np.ascontiguousarray(a[rows]), b, bi)) <= TOL_FP32
+
+
+@pytest.mark.parametrize("n0,n1,K,p2,ne02", [(256, 128, 2601, 1, 1), (33, 32, 4099, 1, 1), (36, 132, 65, 2, 1), (8, 4, 64, 1, 1),
+                                             (130, 66, 1000, 3, 3), (64, 64, 16 * 64 + 1, 1, 1)])
+def test_exact_contraction_split(oracle, n0, n1, K, p2, ne02):
+    """Few output tiles and a long contraction: split over the groups of a CTA and the CTAs of a cluster.  Repeats give the
+    same bits (the parts are added in a fixed order)."""
+    s0, s1 = cases.out_prod_case(n0, n1, K, p2, 1, ne02=ne02, seed=32)
+    got = host(ops.out_prod_cuda(dev(s0), dev(s1), path=PATH_SIMT))
+    assert cases.rel_err(got, oracle.out_prod(s0, s1)) <= TOL_FP32
+    assert np.array_equal(got, host(ops.out_prod_cuda(dev(s0), dev(s1), path=PATH_SIMT)))
+
+
 def test_attention_full_size_properties():
     """The full-size attention case (MSA depth 256, L = 256, 8 heads x 32, shared pair bias): the tensor-core kernel
     agrees with the CUDA-core kernel, a permutation of the batch permutes the output, and exp(LSE) equals the
