@@ -380,6 +380,7 @@ int ppml_b200_out_prod(const float* src0, const float* src1, float* dst,
             a.batch = static_cast<int>(ne2 * ne3);
             a.lda = ne10; a.ldb = ne00; a.a_batch = ne10 * ne11; a.b_batch = ne00 * ne01;
             a.ldc = ne0; a.c_batch = ne0 * ne1; a.alpha = 1.0f; a.elem = 0; a.tf32_mode = PPML_B200_TF32_TMA; a.mn_major = 1;
+            a.may_split = 1;
             rc = launch_umma_gemm(a, as_stream(stream));
         }
         if (rc != ST_UNSUPPORTED_PATH || path == PPML_B200_PATH_UMMA) return rc;

@@ -97,6 +97,7 @@ struct UmmaGemmArgs {
     int tf32_mode;                     // fp32 only: 0 round in smem (rna), 1 TMA tf32 type, 2 truncate
     int mn_major;                      // 1: A[b][k][m], B[b][k][n] (row index contiguous; lda / ldb = k pitch), fp32 only
     const float* ln_stats; const float* ln_u; const float* gate; int act;      // fused LayerNorm algebra / activation gate
+    int may_split;                     // 1: the contraction may be split over CTAs (mn_major, fp32; no bias, no clamp)
 };
 int launch_umma_gemm(const UmmaGemmArgs& a, cudaStream_t st);
 

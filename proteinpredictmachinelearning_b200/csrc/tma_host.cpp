@@ -55,7 +55,8 @@ bool make_tmap_3d(CUtensorMap* out, TmaType type, const void* base, uint64_t d0,
 }
 
 bool make_tmap_4d(CUtensorMap* out, TmaType type, const void* base, uint64_t d0, uint64_t d1, uint64_t d2, uint64_t d3,
-                  uint64_t stride1_bytes, uint64_t stride2_bytes, uint64_t stride3_bytes, uint32_t box0, uint32_t box1, int swizzle) {
+                  uint64_t stride1_bytes, uint64_t stride2_bytes, uint64_t stride3_bytes, uint32_t box0, uint32_t box1, int swizzle,
+                  uint32_t box2) {
     EncodeTiledFn fn = encode_fn();
     if (!fn) return false;
     CUtensorMapDataType dt;
@@ -71,7 +72,7 @@ bool make_tmap_4d(CUtensorMap* out, TmaType type, const void* base, uint64_t d0,
     if (stride3_bytes == 0) stride3_bytes = stride2_bytes * d2;      // a degenerate outer extent still needs a legal stride
     cuuint64_t gdim[4] = {d0, d1, d2, d3};
     cuuint64_t gstride[3] = {stride1_bytes, stride2_bytes, stride3_bytes};
-    cuuint32_t box[4] = {box0, box1, 1, 1};
+    cuuint32_t box[4] = {box0, box1, box2, 1};
     cuuint32_t estr[4] = {1, 1, 1, 1};
     CUresult r = fn(out, dt, 4, const_cast<void*>(base), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                     swizzle == 4 ? CU_TENSOR_MAP_SWIZZLE_32B : swizzle == 3 ? CU_TENSOR_MAP_SWIZZLE_64B : swizzle == 2 ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B

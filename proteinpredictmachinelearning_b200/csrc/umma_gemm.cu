@@ -1,6 +1,7 @@
 // umma_gemm.cu -- host side of the tcgen05 contraction engine: eligibility checks, tensor maps,
 // tile shape selection and the launch.
 #include <cstdlib>
+#include <mutex>
 #include "kernels.h"
 #include "tma_host.h"
 #include "umma_gemm.cuh"
@@ -78,6 +79,75 @@ int launch_bn_mn(int BN, bool half, const CUtensorMap& tmA, const CUtensorMap& t
     }
 }
 
+template <int BN>
+struct SplitGemm {
+    static void config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute& at, unsigned tiles, int splits, cudaStream_t st) {
+        cfg.gridDim = dim3(tiles, static_cast<unsigned>(splits)); cfg.blockDim = dim3(192); cfg.dynamicSmemBytes = gemm_split_smem_bytes<BN>();
+        cfg.stream = st;
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = 1; at.val.clusterDim.y = static_cast<unsigned>(splits); at.val.clusterDim.z = 1;
+        cfg.attrs = &at; cfg.numAttrs = 1;
+    }
+    // clusters of each size that run together on the current device, asked once per device; null on an error
+    static const int (*resident(int dev))[17] {
+        static int table[64][17];
+        static std::once_flag once[64];
+        static bool ok[64];
+        std::call_once(once[dev], [&] {
+            auto kern = umma_gemm_split_kernel<BN>;
+            ok[dev] = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, gemm_split_smem_bytes<BN>()) == cudaSuccess &&
+                      cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+            for (int s = 2; ok[dev] && s <= 16; ++s) {
+                cudaLaunchConfig_t cfg{};
+                cudaLaunchAttribute at{};
+                config(cfg, at, 1, s, nullptr);
+                int n = 0;
+                table[dev][s] = cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess ? n : 0;
+            }
+            cudaGetLastError();
+        });
+        return ok[dev] ? &table[dev] : nullptr;
+    }
+    static int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, GemmParams p, int box_a, int splits, cudaStream_t st) {
+        p.n_tiles = (p.N + BN - 1) / BN;
+        p.m_tiles = (p.M + 127) / 128;
+        cudaLaunchConfig_t cfg{};
+        cudaLaunchAttribute at{};
+        config(cfg, at, static_cast<unsigned>(p.m_tiles * p.n_tiles * p.batch), splits, st);
+        if (cudaLaunchKernelEx(&cfg, umma_gemm_split_kernel<BN>, tmA, tmB, p, box_a) != cudaSuccess) { cudaGetLastError(); return ST_LAUNCH; }
+        return ST_OK;
+    }
+};
+
+// Tile width and cluster size of the split form: the fewest operand bytes one after the other into an SM -- K steps of a CTA times
+// its rows, times the waves of clusters (what does not run together waits).  bn = 0: more than half the SMs have a tile of the
+// general kernel, or there are fewer than four K steps (256 x 256 over 256 tokens, eight of them: 11.7 -> 5.4 us; over 128: 9.4 -> 4.7).
+struct GemmSplit { int bn = 0, splits = 1; };
+template <int BN>
+void plan_gemm_split(GemmSplit& best, long long& cost, int dev, const UmmaGemmArgs& a, int k_steps) {
+    const int (*res)[17] = SplitGemm<BN>::resident(dev);
+    if (!res || (BN > 32 && a.N <= BN / 2)) return;
+    const long long tiles = static_cast<long long>((a.M + 127) / 128) * ((a.N + BN - 1) / BN) * a.batch;
+    const long long rows = (a.M < 128 ? a.M : 128) + (a.N < BN ? a.N : BN);
+    for (int s = 2; s <= 16 && s <= k_steps; ++s) {
+        if ((*res)[s] <= 0) continue;
+        const long long c = ((tiles + (*res)[s] - 1) / (*res)[s]) * ((k_steps + s - 1) / s) * rows;
+        if (c < cost) { cost = c; best.bn = BN; best.splits = s; }
+    }
+}
+GemmSplit gemm_split(const UmmaGemmArgs& a, int general_bn, int k_steps) {
+    GemmSplit g;
+    int dev = 0;
+    if (!a.may_split || k_steps < 4 || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return g;
+    const long long tiles = static_cast<long long>((a.M + 127) / 128) * ((a.N + general_bn - 1) / general_bn) * a.batch;
+    if (2 * tiles > num_sms()) return g;
+    long long cost = static_cast<long long>(k_steps) * (128 + general_bn);
+    plan_gemm_split<128>(g, cost, dev, a, k_steps);
+    plan_gemm_split<64>(g, cost, dev, a, k_steps);
+    plan_gemm_split<32>(g, cost, dev, a, k_steps);
+    return g;
+}
+
 int pick_bn(int N) {
     if (N <= 32) return 32;
     if (N <= 64) return 64;
@@ -121,6 +191,24 @@ int launch_umma_gemm(const UmmaGemmArgs& a, cudaStream_t st) {
         p.bias = a.bias; p.alpha = a.alpha; p.clamp = a.clamp;
         p.err = err;
         p.vec_ok = ((reinterpret_cast<uintptr_t>(a.C) & 15u) == 0) && (a.ldc % 4 == 0) && (a.c_batch % 4 == 0) && (a.N % 4 == 0);
+        const GemmSplit g = half ? GemmSplit() : gemm_split(a, BN, p.k_steps);
+        if (g.bn != 0) {
+            int box_a = 0;
+            // whole row blocks: an operand as [batch][row block][k][32], whose box holds all row blocks of a stage (one
+            // issuing thread needs 60 to 80 ns per load: 256 x 256 over 65536 tokens 62 us with a box per row block)
+            if (a.M % 32 == 0 && a.N % 32 == 0) {
+                const uint32_t ba = a.M < 128 ? a.M / 32 : 4, bb = (a.N < g.bn ? a.N : g.bn) / 32;
+                CUtensorMap wa, wb;
+                if (make_tmap_4d(&wa, tt, a.A, 32, a.K, a.M / 32, a.batch, static_cast<uint64_t>(a.lda) * es, 128, a_bs, 32, 32, 2, ba) &&
+                    make_tmap_4d(&wb, tt, a.B, 32, a.K, a.N / 32, a.batch, static_cast<uint64_t>(a.ldb) * es, 128, b_bs, 32, 32, 2, bb)) {
+                    tmA = wa; tmB = wb;
+                    box_a = static_cast<int>(ba);
+                }
+            }
+            if (g.bn == 128) return SplitGemm<128>::launch(tmA, tmB, p, box_a, g.splits, st);
+            if (g.bn == 64) return SplitGemm<64>::launch(tmA, tmB, p, box_a, g.splits, st);
+            return SplitGemm<32>::launch(tmA, tmB, p, box_a, g.splits, st);
+        }
         return launch_bn_mn(BN, half, tmA, tmB, p, st);
     }
     TmaType tt = (a.elem == 0) ? (a.tf32_mode == 1 ? TmaType::TF32 : TmaType::F32)

@@ -11,6 +11,8 @@
 // TMEM holds two accumulators of BN columns so the epilogue of a tile overlaps the next tile's
 // main loop.  Every wait is bounded (common.cuh).
 #pragma once
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 
 namespace ppml_b200 {
@@ -429,6 +431,153 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     // common exit: all roles meet here (also after an aborted wait) before TMEM is released
     tc_fence_before();
     __syncthreads();
+    if (warp == 1) {
+        tc_fence_after();
+        tmem_dealloc(tmem_base, TMEM_COLS);
+    }
+}
+
+// =============================================================================================
+// The split form for a long contraction with a small result (weight gradients: dW = dY^T X over the tokens), fp32 operands with
+// the row index contiguous.  A cluster of up to 16 CTAs shares one 128 x BN tile: CTA r takes the K steps r, r + S, ...
+// (neighbouring in memory at any time), leaves its accumulator in its shared memory, and the CTAs add the parts piece by piece
+// in rank order over distributed shared memory -- no workspace, no atomics.  Partial sums stay fp32.
+//
+// Bound: operand bytes into each SM -- a CTA reads (128 + BN) * 4 bytes per token it owns, at most 16 CTAs share a tile
+// (64 SMs for 256 x 256: 93 GB/s each).  One CTA per tile, as the general kernel runs it, left 146 SMs idle: 256 x 256 over
+// 65536 tokens 1181 -> 45 us (134 MB: 21 us at copy bandwidth), 64 x 32 747 -> 41, 256 x 128 over 2601 41 -> 7.5.
+// =============================================================================================
+template <int BN>
+__host__ __device__ constexpr int gemm_split_smem_bytes() { return gemm_num_stages<BN>() * gemm_stage_bytes<BN>() + 1024 + 512; }
+
+template <int BN>
+__global__ void __launch_bounds__(192, 1)
+umma_gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmParams p,
+                       int box_a /* row blocks of 32 in a 4-D box of A (both maps are 4-D then); 0: 3-D maps, a box per row block */) {
+    constexpr int STAGES = gemm_num_stages<BN>();
+    constexpr int STAGE_BYTES = gemm_stage_bytes<BN>();
+    constexpr int BK = 32, kBox = BK * 128;
+    constexpr int kPitch = BN + 4;                        // floats per row of the partial tile: 16-byte writes of 8 rows hit 8 bank groups
+    constexpr uint32_t TMEM_COLS = BN < 32 ? 32 : BN;
+    static_assert(128 * kPitch * 4 <= STAGES * STAGE_BYTES, "the partial tile reuses the stages");
+
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));       // the same offset in every CTA of the cluster
+    const uint32_t bar_base = smem_base + STAGES * STAGE_BYTES;
+    auto full_bar = [&](int s) { return bar_base + 8u * s; };
+    auto empty_bar = [&](int s) { return bar_base + 8u * (kGemmMaxStages + s); };
+    const uint32_t done_bar = bar_base + 8u * (2 * kGemmMaxStages);
+    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + STAGES * STAGE_BYTES + 8 * (2 * kGemmMaxStages + 1));
+    volatile int* cta_abort = reinterpret_cast<volatile int*>(smem_gen + STAGES * STAGE_BYTES + 8 * (2 * kGemmMaxStages + 1) + 8);
+
+    namespace cg = cooperative_groups;
+    cg::cluster_group cl = cg::this_cluster();
+    const int splits = static_cast<int>(cl.num_blocks()), rank = static_cast<int>(cl.block_rank());
+    const int warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < STAGES; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
+        mbar_init(done_bar, 1);
+        *cta_abort = 0;
+        fence_barrier_init();
+    }
+    if (warp == 1) {
+        tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), TMEM_COLS);
+        tmem_relinquish();
+    }
+    if (warp == 0 && lane == 0) { prefetch_tmap(&tmA); prefetch_tmap(&tmB); }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+
+    const int tile = blockIdx.x, tiles_per_batch = p.m_tiles * p.n_tiles;
+    const int b = tile / tiles_per_batch, r_ = tile - b * tiles_per_batch;
+    const int mt = r_ / p.n_tiles, nt = r_ - mt * p.n_tiles;
+    const int row0 = mt * 128, col0 = nt * BN;
+
+    if (warp == 0) {
+        if (lane == 0) {
+            // only boxes that hold rows of the operand: what the others' part of the stage contains reaches only accumulator rows
+            // and columns outside the result
+            const int na = box_a ? box_a : min(128 / BK, (p.M - row0 + BK - 1) / BK);
+            const int nb = box_a ? min(BN, p.N) / BK : min(BN / BK, (p.N - col0 + BK - 1) / BK);
+            uint32_t it = 0;
+            for (int ks = rank; ks < p.k_steps; ks += splits, ++it) {
+                const int s = it % STAGES;
+                if (!mbar_wait(empty_bar(s), ((it / STAGES) & 1u) ^ 1u, cta_abort, p.err, 0x111)) break;
+                const uint32_t sa = smem_base + s * STAGE_BYTES;
+                mbar_arrive_expect_tx(full_bar(s), static_cast<uint32_t>(na + nb) * kBox);
+                if (box_a) {                             // all row blocks of an operand with one instruction
+                    tma_load_4d(sa, &tmA, full_bar(s), 0, ks * BK, row0 / BK, b);
+                    tma_load_4d(sa + kGemmStageA, &tmB, full_bar(s), 0, ks * BK, col0 / BK, b);
+                    continue;
+                }
+                for (int i = 0; i < na; ++i) tma_load_3d(sa + i * kBox, &tmA, full_bar(s), row0 + i * BK, ks * BK, b);
+                for (int i = 0; i < nb; ++i) tma_load_3d(sa + kGemmStageA + i * kBox, &tmB, full_bar(s), col0 + i * BK, ks * BK, b);
+            }
+        }
+        __syncwarp();
+    } else if (warp == 1) {
+        if (lane == 0) {
+            const uint32_t idesc = make_idesc(1, 2, 2, 1, 1, 128, BN);
+            uint32_t it = 0;
+            bool ok = true;
+            for (int ks = rank; ks < p.k_steps; ks += splits, ++it) {
+                const int s = it % STAGES;
+                if (!mbar_wait(full_bar(s), (it / STAGES) & 1u, cta_abort, p.err, 0x212)) { ok = false; break; }
+                tc_fence_after();
+                const uint32_t sa = smem_base + s * STAGE_BYTES;
+                const uint64_t da = make_smem_desc(sa, BK * 128, 512, kLayoutSW128Base32);
+                const uint64_t db = make_smem_desc(sa + kGemmStageA, BK * 128, 512, kLayoutSW128Base32);
+#pragma unroll
+                for (int kk = 0; kk < 4; ++kk)
+                    umma<MmaKind::TF32>(tmem_base, da + 64u * kk, db + 64u * kk, idesc, (it | kk) != 0 ? 1u : 0u);
+                umma_commit(empty_bar(s));
+            }
+            if (ok) umma_commit(done_bar);
+        }
+        __syncwarp();
+    } else {
+        // accumulator -> this CTA's partial tile [128][kPitch] (thread = row), over the stages: every load has been consumed
+        const int q = warp & 3;
+        if (mbar_wait(done_bar, 0, cta_abort, p.err, 0x313)) {
+            tc_fence_after();
+            float* row = reinterpret_cast<float*>(smem_gen) + (q * 32 + lane) * kPitch;
+#pragma unroll 1
+            for (int c = 0; c < BN / 32; ++c) {
+                uint32_t v[32];
+                tmem_ld32(tmem_base + c * 32 + (static_cast<uint32_t>(q * 32) << 16), v);
+                tmem_ld_wait();
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    *reinterpret_cast<uint4*>(row + c * 32 + j * 4) = make_uint4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+            }
+        }
+        tc_fence_before();
+    }
+    cl.sync();                                            // every part is in place (also after an aborted wait)
+    float* C = p.C + static_cast<long long>(b) * p.c_batch;
+    for (int e = rank * 192 + static_cast<int>(threadIdx.x); e < 128 * BN / 4; e += splits * 192) {
+        const int r = e / (BN / 4), c = (e % (BN / 4)) * 4;
+        if (row0 + r >= p.M || col0 + c >= p.N) continue;
+        float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int k = 0; k < splits; ++k) {
+            const float4 x = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(cl.map_shared_rank(smem_gen, k)) + r * kPitch + c);
+            s.x += x.x; s.y += x.y; s.z += x.z; s.w += x.w;
+        }
+        s.x *= p.alpha; s.y *= p.alpha; s.z *= p.alpha; s.w *= p.alpha;
+        float* dst = C + static_cast<long long>(row0 + r) * p.ldc + col0 + c;
+        if (p.vec_ok) *reinterpret_cast<float4*>(dst) = s;
+        else {
+            dst[0] = s.x;
+            if (col0 + c + 1 < p.N) dst[1] = s.y;
+            if (col0 + c + 2 < p.N) dst[2] = s.z;
+            if (col0 + c + 3 < p.N) dst[3] = s.w;
+        }
+    }
+    cl.sync();                                            // nobody leaves while a peer still reads
     if (warp == 1) {
         tc_fence_after();
         tmem_dealloc(tmem_base, TMEM_COLS);

@@ -799,6 +799,17 @@ def test_exact_contraction_split(oracle, n0, n1, K, p2, ne02):
     assert np.array_equal(got, host(ops.out_prod_cuda(dev(s0), dev(s1), path=PATH_SIMT)))
 
 
+@pytest.mark.parametrize("n0,n1,K,p2", [(256, 128, 2601, 1), (64, 256, 4096, 1), (36, 20, 300, 1), (100, 36, 1000, 1), (64, 160, 225, 2),
+                                        (32, 32, 128, 1), (256, 256, 97, 1), (4, 4, 5000, 1), (260, 132, 700, 1)])
+def test_out_prod_split_on_tensor_cores(oracle, n0, n1, K, p2):
+    """Weight-gradient shapes: few output tiles, the contraction shared by a cluster (whole row blocks and ragged ones, K tails,
+    one CTA with a single step).  Repeats give the same bits."""
+    s0, s1 = cases.out_prod_case(n0, n1, K, p2, 1, seed=33)
+    got = host(ops.out_prod_cuda(dev(s0), dev(s1), path=PATH_UMMA))
+    assert cases.rel_err(got, oracle.out_prod(s0, s1)) <= TOL_TF32
+    assert np.array_equal(got, host(ops.out_prod_cuda(dev(s0), dev(s1), path=PATH_UMMA)))
+
+
 def test_attention_full_size_properties():
     """The full-size attention case (MSA depth 256, L = 256, 8 heads x 32, shared pair bias): the tensor-core kernel
     agrees with the CUDA-core kernel, a permutation of the batch permutes the output, and exp(LSE) equals the
