@@ -121,7 +121,7 @@ struct Loader<T, Fetch::ANY, ROWS, NT> {
 
 // One slice of a warp's 32 x 8 TN outputs: lane rows {arow .. +3, arow + 16 ..}, lane columns {bcol .. +3 (, bcol + 32 ..)}.  Per k
 // two 16-byte reads of A (four distinct addresses in the warp) and TN / 4 of B (eight) feed 8 TN FMAs.  The FMAs are packed pairs
-// of columns: a pair takes the FMA pipe as long as two scalar ones but one issue slot, which leaves slots for the reads
+// of rows: a pair takes the FMA pipe as long as two scalar ones but one issue slot, which leaves slots for the reads
 // (4096 x 4096 x 4096: 41 TFLOP/s with scalar FMAs, 52 packed; the same rounding either way).
 template <Fetch F, int BM, int BN, int TN>
 __device__ __forceinline__ void mac_slice(const float* as, const float* bs, int arow, int bcol, float (&acc)[8][TN]) {
@@ -133,15 +133,12 @@ __device__ __forceinline__ void mac_slice(const float* as, const float* bs, int 
         *reinterpret_cast<float4*>(a + 4) = *reinterpret_cast<const float4*>(as + kk * BM + ((arow + 16) ^ sw));
         *reinterpret_cast<float4*>(b) = *reinterpret_cast<const float4*>(bs + kk * BN + (bcol ^ sw));
         if constexpr (TN == 8) *reinterpret_cast<float4*>(b + 4) = *reinterpret_cast<const float4*>(bs + kk * BN + ((bcol + 32) ^ sw));
-        uint64_t b2[TN / 2];
 #pragma unroll
-        for (int j = 0; j < TN / 2; ++j) b2[j] = pack2(b[2 * j], b[2 * j + 1]);
+        for (int j = 0; j < TN; ++j) {
+            const uint64_t b2 = pack2(b[j], b[j]);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const uint64_t a2 = pack2(a[i], a[i]);
-#pragma unroll
-            for (int j = 0; j < TN / 2; ++j)
-                unpack2(ffma2(a2, b2[j], pack2(acc[i][2 * j], acc[i][2 * j + 1])), acc[i][2 * j], acc[i][2 * j + 1]);
+            for (int i = 0; i < 8; i += 2)
+                unpack2(ffma2(pack2(a[i], a[i + 1]), b2, pack2(acc[i][j], acc[i + 1][j])), acc[i][j], acc[i + 1][j]);
         }
     }
 }
