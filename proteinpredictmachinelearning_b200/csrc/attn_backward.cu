@@ -6,28 +6,26 @@
 //
 // Two kernels, each recomputing the scores of its tiles (nothing but the outputs is written, every output element is
 // written exactly once, so no zero-fill pass and no atomic adds: the results do not depend on the launch order):
-//   attn_bwd_dq_kernel   one CTA = 32 query rows of one (batch, head); walks the key tiles of 32; writes dQ and dbias
-//   attn_bwd_dkv_kernel  one CTA = 32 key rows of one (batch, head); walks the query tiles of 32; writes dK and dV
-// In both, a warp owns 8 rows of the CTA's 32.  Per tile of 32 partner rows it works in two phases:
-//   1. lane = partner row: dot products over d against the warp's rows (own rows broadcast from shared memory, partner
-//      rows read from padded tiles), exp, dS; dS (and P) go to a small shared buffer, dbias to global memory (coalesced);
-//   2. lane = channel d: accumulates its channel of the 8 rows over the 32 partners (dS broadcast, partner tile read
-//      along d), one register per row and channel -- no cross-lane reduction.
+//   attn_bwd_dq_kernel   one CTA = 64 query rows of one (batch, head); walks the key tiles of 64; writes dQ and dbias
+//   attn_bwd_dkv_kernel  one CTA = 64 key rows of one (batch, head); walks the query tiles of 64; writes dK and dV
+// Per tile: scores and dP as register tiles over the channels, exp and dS in registers, dS (and P, one after the other through
+// the same buffer) to shared memory as [partner][own row], then the result's register tile over the partners (attn_tile.cuh).
+//
+// Bound: instruction issue (fp32 FMAs are half of it: 3 products in one kernel, 4 in the other; FMA pipe 45 % busy at two CTAs
+// per SM).  64 x 8 x 256 x 32 with dbias 1535 -> 510 us (30 TFLOP/s over the seven products), head dim 8 613 -> 259 us, against the form with a warp per 8 rows, whose lanes read one scalar from shared memory per FMA or two.  The next
+// tile and this tile's bias are requested before the products (255 registers, two CTAs per SM): 573 us with three CTAs per SM
+// that wait for them.
 // Layouts as the forward: Q, K, V, O, dO, dQ, dK, dV [B, h, L, d]; bias [B, h, L, L] with a batch stride (0: shared);
 // dbias [B, h, L, L]; LSE [B, h, L].  d <= 64.
 #include <cuda_runtime.h>
 #include <math_constants.h>
 
-#include "common.cuh"
+#include "attn_tile.cuh"
 #include "kernels.h"
 
 namespace ppml_b200 {
 
 namespace {
-
-constexpr int kRows = 32;        // rows of a CTA (query rows / key rows) = partner rows of a tile
-constexpr int kWarps = 4;
-constexpr int kRpw = kRows / kWarps;   // rows per warp
 
 struct BwdParams {
     int B, H, L, d, causal;
@@ -35,249 +33,302 @@ struct BwdParams {
     const float *Q, *K, *V, *bias, *O, *dO, *LSE;
     long long bias_batch_stride;
     float *dQ, *dK, *dV, *dbias;
+    int vec_in;             // rows of Q, K, V, O, dO in 16-byte pieces
+    int vec_out;            // rows of dQ, dK, dV
+    int vec_bias;           // rows of bias; vec_dbias: rows of dbias
+    int vec_dbias;
 };
 
-// rows [r0, r0 + 32) of a [L][d] matrix into a padded shared tile [32][DP + 1] (rows past L and channels past d: 0)
+constexpr int kT = kAttnTile;
+
+// D_i of the 64 query rows whose dO and O rows are in registers: a row lies in DP / 4 neighbouring lanes
 template <int DP>
-__device__ __forceinline__ void load_tile(float* dst, const float* src, int r0, int L, int d) {
-    for (int idx = threadIdx.x; idx < kRows * DP; idx += kWarps * 32) {
-        const int r = idx / DP, c = idx - r * DP;
-        dst[r * (DP + 1) + c] = (r0 + r < L && c < d) ? src[static_cast<size_t>(r0 + r) * d + c] : 0.0f;
+__device__ __forceinline__ void store_row_dots(const AttnRows<DP>& g, const AttnRows<DP>& o, float* Dr) {
+#pragma unroll
+    for (int it = 0; it < AttnRows<DP>::kN; ++it) {
+        const float4 a = g.v[it], b = o.v[it];
+        float D = fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, a.x * b.x)));
+#pragma unroll
+        for (int off = 1; off < DP / 4; off <<= 1) D += __shfl_xor_sync(0xffffffffu, D, off);
+        if (AttnRows<DP>::chan() == 0) Dr[AttnRows<DP>::row(it)] = D;
+    }
+}
+// LSE of query row i0 + thread (threads of the first 64); rows past L: -inf, which masks them
+__device__ __forceinline__ float row_lse(const BwdParams& p, int bh, int i0) {
+    const int i = i0 + static_cast<int>(threadIdx.x);
+    return (threadIdx.x < kT && i < p.L) ? p.LSE[static_cast<size_t>(bh) * p.L + i] : -CUDART_INF_F;
+}
+
+// rows [r0, r0 + 64) of a result from the groups' parts
+template <int DP>
+__device__ __forceinline__ void store_rows(float* dst, const float* red, int r0, int L, int d, float scale, bool vec) {
+    for (int e = threadIdx.x; e < kT * DP / 4; e += kAttnThreads) {
+        const int r = e / (DP / 4), c = (e % (DP / 4)) * 4;
+        if (r0 + r >= L || c >= d) continue;
+        const float4 s = AttnOut<DP>::sum(red, r, c);
+        float* o = dst + static_cast<size_t>(r0 + r) * d + c;
+        if (vec) *reinterpret_cast<float4*>(o) = make_float4(scale * s.x, scale * s.y, scale * s.z, scale * s.w);
+        else {
+            o[0] = scale * s.x;
+            if (c + 1 < d) o[1] = scale * s.y;
+            if (c + 2 < d) o[2] = scale * s.z;
+            if (c + 3 < d) o[3] = scale * s.w;
+        }
     }
 }
 
-// ---- dQ and dbias -------------------------------------------------------------------------------------------------------
-template <int DP>
-__global__ void __launch_bounds__(kWarps * 32) attn_bwd_dq_kernel(const BwdParams p) {
-    extern __shared__ float sm[];
-    float* Ks = sm;                                   // [32][DP + 1]
-    float* Vs = Ks + kRows * (DP + 1);                // [32][DP + 1]
-    float* Qs = Vs + kRows * (DP + 1);                // [32][DP]   this CTA's query rows
-    float* dOs = Qs + kRows * DP;                     // [32][DP]
-    float* dS = dOs + kRows * DP;                     // [kWarps][32 partners][kRpw]
-    float* Dr = dS + kWarps * 32 * kRpw;              // [32]  D_i
-    float* Ls = Dr + kRows;                           // [32]  LSE_i
+// four neighbours of a row of [L] floats from column c on, or `fill` past L
+__device__ __forceinline__ float4 row4(const float* row, int c, int L, bool vec) {
+    if (vec) return c < L ? attn_ld4(row + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (c < L) v.x = row[c];
+    if (c + 1 < L) v.y = row[c + 1];
+    if (c + 2 < L) v.z = row[c + 2];
+    if (c + 3 < L) v.w = row[c + 3];
+    return v;
+}
+__device__ __forceinline__ void put4(float* row, int c, int L, bool vec, const float (&v)[4]) {
+    if (vec) { if (c < L) *reinterpret_cast<float4*>(row + c) = make_float4(v[0], v[1], v[2], v[3]); return; }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) if (c + j < L) row[c + j] = v[j];
+}
 
-    const int bh = blockIdx.y, i0 = blockIdx.x * kRows;
+// ---- dQ and dbias -------------------------------------------------------------------------------------------------------
+template <int DP> constexpr int dq_smem_floats() { return 5 * DP * kT + kT * kT + 2 * kT; }
+
+template <int DP>
+__global__ void __launch_bounds__(kAttnThreads, 2) attn_bwd_dq_kernel(const BwdParams p) {
+    extern __shared__ __align__(16) float sm[];
+    float* Qt = sm;                                   // own rows, transposed
+    float* dOt = Qt + DP * kT;
+    float* Kt = dOt + DP * kT;                        // key tile, transposed
+    float* Vt = Kt + DP * kT;
+    float* Kr = Vt + DP * kT;                         // key tile, row by row
+    float* probs = Kr + DP * kT;                      // dS [key][query]
+    float* Dr = probs + kT * kT;
+    float* Ls = Dr + kT;
+
+    const int bh = blockIdx.y, i0 = blockIdx.x * kT;
     const int b = bh / p.H, hh = bh - b * p.H;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int arow = (warp >> 1) * 32 + ((lane & 1) | ((lane >> 4) << 1)) * 4, bcol = (warp & 1) * 32 + ((lane >> 1) & 7) * 4;
     const size_t base = static_cast<size_t>(bh) * p.L * p.d;
     const float* bias = p.bias ? p.bias + static_cast<size_t>(b) * p.bias_batch_stride + static_cast<size_t>(hh) * p.L * p.L : nullptr;
     float* dbias = p.dbias ? p.dbias + static_cast<size_t>(bh) * p.L * p.L : nullptr;
 
-    // this CTA's rows: Q, dO (unpadded rows: they are read as broadcasts), D_i, LSE_i
-    for (int idx = threadIdx.x; idx < kRows * DP; idx += kWarps * 32) {
-        const int r = idx / DP, c = idx - r * DP;
-        const bool in = i0 + r < p.L && c < p.d;
-        Qs[idx] = in ? p.Q[base + static_cast<size_t>(i0 + r) * p.d + c] : 0.0f;
-        dOs[idx] = in ? p.dO[base + static_cast<size_t>(i0 + r) * p.d + c] : 0.0f;
+    AttnRows<DP> rk, rv;                              // the next key tile on its way
+    {
+        AttnRows<DP> q, g, o;
+        q.fetch(p.Q + base, p.d, i0, p.L, p.d, p.vec_in);
+        g.fetch(p.dO + base, p.d, i0, p.L, p.d, p.vec_in);
+        o.fetch(p.O + base, p.d, i0, p.L, p.d, p.vec_in);
+        const float lse = row_lse(p, bh, i0);
+        rk.fetch(p.K + base, p.d, 0, p.L, p.d, p.vec_in);
+        rv.fetch(p.V + base, p.d, 0, p.L, p.d, p.vec_in);
+        q.template store<true, false>(Qt, nullptr);
+        g.template store<true, false>(dOt, nullptr);
+        store_row_dots<DP>(g, o, Dr);
+        if (threadIdx.x < kT) Ls[threadIdx.x] = lse;
     }
-    if (threadIdx.x < kRows) {
-        const int i = i0 + threadIdx.x;
-        float D = 0.0f, lse = -CUDART_INF_F;
-        if (i < p.L) {
-            lse = p.LSE[static_cast<size_t>(bh) * p.L + i];
-            for (int c = 0; c < p.d; ++c) D += p.dO[base + static_cast<size_t>(i) * p.d + c] * p.O[base + static_cast<size_t>(i) * p.d + c];
-        }
-        Dr[threadIdx.x] = D; Ls[threadIdx.x] = lse;
-    }
-    __syncthreads();
 
-    constexpr int NACC = (DP + 31) / 32;              // channels per lane in phase 2
-    float acc[kRpw][NACC];
+    const AttnOut<DP> out;
+    float o[8][AttnOut<DP>::kCols];
 #pragma unroll
-    for (int r = 0; r < kRpw; ++r)
+    for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int a = 0; a < NACC; ++a) acc[r][a] = 0.0f;
+        for (int c = 0; c < AttnOut<DP>::kCols; ++c) o[i][c] = 0.0f;
 
-    const int jend = p.causal ? min(p.L, i0 + kRows) : p.L;      // keys past the last row's diagonal are masked for all
-    float* dSw = dS + warp * 32 * kRpw;
-    for (int j0 = 0; j0 < jend; j0 += kRows) {
+    const int jend = p.causal ? min(p.L, i0 + kT) : p.L;         // keys past the last row's diagonal are masked for all
+    for (int j0 = 0; j0 < jend; j0 += kT) {
         __syncthreads();                               // the tiles of the previous step are no longer read
-        load_tile<DP>(Ks, p.K + base, j0, p.L, p.d);
-        load_tile<DP>(Vs, p.V + base, j0, p.L, p.d);
+        rk.template store<true, true>(Kt, Kr);
+        rv.template store<true, false>(Vt, nullptr);
+        const int j = j0 + bcol;
+        float4 bi[8];                                  // this tile's bias and the next tile's keys travel during the products
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+            const int i = i0 + arow + (r < 4 ? r : 12 + r);
+            bi[r] = (bias && i < p.L) ? row4(bias + static_cast<size_t>(i) * p.L, j, p.L, p.vec_bias) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        if (j0 + kT < jend) {
+            rk.fetch(p.K + base, p.d, j0 + kT, p.L, p.d, p.vec_in);
+            rv.fetch(p.V + base, p.d, j0 + kT, p.L, p.d, p.vec_in);
+        }
         __syncthreads();
-        // phase 1: lane = key j0 + lane, against the warp's 8 query rows
-        const int j = j0 + lane;
-        const float* kr = Ks + lane * (DP + 1);
-        const float* vr = Vs + lane * (DP + 1);
+        float s[8][4], dp[8][4];
+        attn_scores<DP, 16>(Qt, Kt, arow, bcol, s);
+        attn_scores<DP, 16>(dOt, Vt, arow, bcol, dp);
 #pragma unroll
-        for (int r = 0; r < kRpw; ++r) {
-            const int rl = warp * kRpw + r, i = i0 + rl;
-            const float* q = Qs + rl * DP;
-            const float* go = dOs + rl * DP;
-            float s = 0.0f, dp = 0.0f;
-#pragma unroll 8
-            for (int c = 0; c < DP; ++c) { s = fmaf(q[c], kr[c], s); dp = fmaf(go[c], vr[c], dp); }
-            const float lse = Ls[rl];
-            float ds = 0.0f;
-            const bool live = i < p.L && j < p.L && (!p.causal || j <= i) && lse > -CUDART_INF_F;
-            if (live) {
-                s *= p.scale;
-                if (bias) s += bias[static_cast<size_t>(i) * p.L + j];
-                ds = expf(s - lse) * (dp - Dr[rl]);
+        for (int r = 0; r < 8; ++r) {
+            const int rl = arow + (r < 4 ? r : 12 + r), i = i0 + rl;
+            const float lse = Ls[rl], Di = Dr[rl];
+            const float bj[4] = {bi[r].x, bi[r].y, bi[r].z, bi[r].w};
+            const int keys = (lse > -CUDART_INF_F ? (p.causal ? min(i + 1, p.L) : p.L) : 0) - j;      // visible ones from column j on
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                s[r][u] = u < keys ? expf(s[r][u] * p.scale + bj[u] - lse) * (dp[r][u] - Di) : 0.0f;
             }
-            dSw[lane * kRpw + r] = ds;
-            if (dbias && i < p.L && j < p.L) dbias[static_cast<size_t>(i) * p.L + j] = ds;
+            if (dbias && i < p.L) put4(dbias + static_cast<size_t>(i) * p.L, j, p.L, p.vec_dbias, s[r]);
         }
-        __syncwarp();
-        // phase 2: lane = channel; dQ[i][c] += dS[i][j] K[j][c] over the 32 keys of the tile
-#pragma unroll 4
-        for (int jj = 0; jj < kRows; ++jj) {
-            float dsr[kRpw];
-#pragma unroll
-            for (int r = 0; r < kRpw; ++r) dsr[r] = dSw[jj * kRpw + r];
-#pragma unroll
-            for (int a = 0; a < NACC; ++a) {
-                const int c = lane + 32 * a;
-                const float kv = (c < DP) ? Ks[jj * (DP + 1) + c] : 0.0f;
-#pragma unroll
-                for (int r = 0; r < kRpw; ++r) acc[r][a] = fmaf(dsr[r], kv, acc[r][a]);
-            }
+        if (p.dQ) {
+            attn_store_probs<16>(probs, arow, bcol, s);
+            __syncthreads();
+            out.mac(probs, Kr, o);
         }
-        __syncwarp();
     }
     // keys past jend of a causal CTA: dbias stays 0 there
     if (dbias && p.causal) {
-        for (int r = 0; r < kRpw; ++r) {
-            const int i = i0 + warp * kRpw + r;
-            if (i < p.L) for (int j = jend + lane; j < p.L; j += 32) dbias[static_cast<size_t>(i) * p.L + j] = 0.0f;
-        }
+        const int j1 = ((jend + kT - 1) / kT) * kT;    // the walked tiles wrote up to here
+        for (int r = warp; r < kT; r += 4)
+            if (i0 + r < p.L) for (int j = j1 + lane; j < p.L; j += 32) dbias[static_cast<size_t>(i0 + r) * p.L + j] = 0.0f;
     }
     if (p.dQ) {
-#pragma unroll
-        for (int r = 0; r < kRpw; ++r) {
-            const int i = i0 + warp * kRpw + r;
-#pragma unroll
-            for (int a = 0; a < NACC; ++a) {
-                const int c = lane + 32 * a;
-                if (i < p.L && c < p.d) p.dQ[base + static_cast<size_t>(i) * p.d + c] = p.scale * acc[r][a];
-            }
-        }
+        __syncthreads();
+        out.spill(probs, o);
+        __syncthreads();
+        store_rows<DP>(p.dQ + base, probs, i0, p.L, p.d, p.scale, p.vec_out);
     }
 }
 
 // ---- dK and dV ----------------------------------------------------------------------------------------------------------
-template <int DP>
-__global__ void __launch_bounds__(kWarps * 32) attn_bwd_dkv_kernel(const BwdParams p) {
-    extern __shared__ float sm[];
-    float* Qs = sm;                                   // [32][DP + 1]  query tile (partner rows)
-    float* dOs = Qs + kRows * (DP + 1);               // [32][DP + 1]
-    float* Ks = dOs + kRows * (DP + 1);               // [32][DP]   this CTA's key rows
-    float* Vs = Ks + kRows * DP;                      // [32][DP]
-    float* dS = Vs + kRows * DP;                      // [kWarps][32 partners][kRpw]
-    float* Ps = dS + kWarps * 32 * kRpw;              // [kWarps][32 partners][kRpw]
-    float* Dr = Ps + kWarps * 32 * kRpw;              // [32]  D_i of the query tile
-    float* Ls = Dr + kRows;                           // [32]  LSE_i of the query tile
+template <int DP> constexpr int dkv_smem_floats() { return 6 * DP * kT + kT * kT + 2 * kT; }
 
-    const int bh = blockIdx.y, j0 = blockIdx.x * kRows;
+template <int DP>
+__global__ void __launch_bounds__(kAttnThreads, 2) attn_bwd_dkv_kernel(const BwdParams p) {
+    extern __shared__ __align__(16) float sm[];
+    float* Kt = sm;                                   // own rows, transposed
+    float* Vt = Kt + DP * kT;
+    float* Qt = Vt + DP * kT;                         // query tile, transposed
+    float* dOt = Qt + DP * kT;
+    float* Qr = dOt + DP * kT;                        // query tile, row by row
+    float* dOr = Qr + DP * kT;
+    float* probs = dOr + DP * kT;                     // P, then dS [query][key]
+    float* Dr = probs + kT * kT;
+    float* Ls = Dr + kT;
+
+    const int bh = blockIdx.y, j0 = blockIdx.x * kT;
     const int b = bh / p.H, hh = bh - b * p.H;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int arow = (warp >> 1) * 32 + ((lane & 1) | ((lane >> 4) << 1)) * 4, bcol = (warp & 1) * 32 + ((lane >> 1) & 7) * 4;
     const size_t base = static_cast<size_t>(bh) * p.L * p.d;
     const float* bias = p.bias ? p.bias + static_cast<size_t>(b) * p.bias_batch_stride + static_cast<size_t>(hh) * p.L * p.L : nullptr;
 
-    for (int idx = threadIdx.x; idx < kRows * DP; idx += kWarps * 32) {
-        const int r = idx / DP, c = idx - r * DP;
-        const bool in = j0 + r < p.L && c < p.d;
-        Ks[idx] = in ? p.K[base + static_cast<size_t>(j0 + r) * p.d + c] : 0.0f;
-        Vs[idx] = in ? p.V[base + static_cast<size_t>(j0 + r) * p.d + c] : 0.0f;
+    const int ibeg = p.causal ? j0 : 0;                // query rows before the first key of the tile see none of it
+    AttnRows<DP> rq, rg, ro;                           // the next query tile on its way: Q, dO, O and the LSE
+    float rl;
+    auto fetch_queries = [&](int i0) {
+        rq.fetch(p.Q + base, p.d, i0, p.L, p.d, p.vec_in);
+        rg.fetch(p.dO + base, p.d, i0, p.L, p.d, p.vec_in);
+        ro.fetch(p.O + base, p.d, i0, p.L, p.d, p.vec_in);
+        rl = row_lse(p, bh, i0);
+    };
+    {
+        AttnRows<DP> k, v;
+        k.fetch(p.K + base, p.d, j0, p.L, p.d, p.vec_in);
+        v.fetch(p.V + base, p.d, j0, p.L, p.d, p.vec_in);
+        fetch_queries(ibeg);
+        k.template store<true, false>(Kt, nullptr);
+        v.template store<true, false>(Vt, nullptr);
     }
 
-    constexpr int NACC = (DP + 31) / 32;
-    float ak[kRpw][NACC], av[kRpw][NACC];
+    const AttnOut<DP> out;
+    constexpr int NC = AttnOut<DP>::kCols;
+    float ok[8][NC], ov[8][NC];
 #pragma unroll
-    for (int r = 0; r < kRpw; ++r)
+    for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int a = 0; a < NACC; ++a) { ak[r][a] = 0.0f; av[r][a] = 0.0f; }
+        for (int c = 0; c < NC; ++c) { ok[i][c] = 0.0f; ov[i][c] = 0.0f; }
 
-    const int ibeg = p.causal ? (j0 / kRows) * kRows : 0;        // query rows before the first key of the tile see none of it
-    float* dSw = dS + warp * 32 * kRpw;
-    float* Pw = Ps + warp * 32 * kRpw;
-    for (int i0 = ibeg; i0 < p.L; i0 += kRows) {
+    for (int i0 = ibeg; i0 < p.L; i0 += kT) {
+        __syncthreads();                               // the tiles of the previous step are no longer read
+        rq.template store<true, true>(Qt, Qr);
+        rg.template store<true, true>(dOt, dOr);
+        store_row_dots<DP>(rg, ro, Dr);
+        if (threadIdx.x < kT) Ls[threadIdx.x] = rl;
+        float4 bi[4][2];                               // this tile's bias and the next query tile travel during the products
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int i = i0 + bcol + u;
+                bi[u][h] = (bias && i < p.L) ? row4(bias + static_cast<size_t>(i) * p.L, j0 + arow + 16 * h, p.L, p.vec_bias)
+                                               : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+        if (i0 + kT < p.L) fetch_queries(i0 + kT);
         __syncthreads();
-        load_tile<DP>(Qs, p.Q + base, i0, p.L, p.d);
-        load_tile<DP>(dOs, p.dO + base, i0, p.L, p.d);
-        if (threadIdx.x < kRows) {
-            const int i = i0 + threadIdx.x;
-            float D = 0.0f, lse = -CUDART_INF_F;
-            if (i < p.L) {
-                lse = p.LSE[static_cast<size_t>(bh) * p.L + i];
-                for (int c = 0; c < p.d; ++c) D += p.dO[base + static_cast<size_t>(i) * p.d + c] * p.O[base + static_cast<size_t>(i) * p.d + c];
+        float s[8][4], dp[8][4];
+        attn_scores<DP, 16>(Kt, Qt, arow, bcol, s);    // [key][query]
+        const float4 l4 = attn_ld4(Ls + bcol);
+        const float lse[4] = {l4.x, l4.y, l4.z, l4.w};
+        int keys[4];                                   // per query: its visible keys from this thread's first key row on
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int i = i0 + bcol + u;
+            keys[u] = (lse[u] > -CUDART_INF_F ? (p.causal ? min(i + 1, p.L) : p.L) : 0) - (j0 + arow);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const float bj[4] = {bi[u][h].x, bi[u][h].y, bi[u][h].z, bi[u][h].w};
+#pragma unroll
+                for (int r = 0; r < 4; ++r)
+                    s[4 * h + r][u] = 16 * h + r < keys[u] ? expf(s[4 * h + r][u] * p.scale + bj[r] - lse[u]) : 0.0f;
             }
-            Dr[threadIdx.x] = D; Ls[threadIdx.x] = lse;
         }
+        attn_store_probs<16>(probs, arow, bcol, s);
+        attn_scores<DP, 16>(Vt, dOt, arow, bcol, dp);
+        const float4 d4 = attn_ld4(Dr + bcol);
+        const float Di[4] = {d4.x, d4.y, d4.z, d4.w};
+#pragma unroll
+        for (int r = 0; r < 8; ++r)
+#pragma unroll
+            for (int u = 0; u < 4; ++u) s[r][u] = (r < 4 ? r : 12 + r) < keys[u] ? s[r][u] * (dp[r][u] - Di[u]) : 0.0f;
         __syncthreads();
-        // phase 1: lane = query i0 + lane, against the warp's 8 key rows
-        const int i = i0 + lane;
-        const float* qr = Qs + lane * (DP + 1);
-        const float* gr = dOs + lane * (DP + 1);
-        const float lse = Ls[lane], Di = Dr[lane];
-#pragma unroll
-        for (int r = 0; r < kRpw; ++r) {
-            const int rl = warp * kRpw + r, j = j0 + rl;
-            const float* k = Ks + rl * DP;
-            const float* v = Vs + rl * DP;
-            float s = 0.0f, dp = 0.0f;
-#pragma unroll 8
-            for (int c = 0; c < DP; ++c) { s = fmaf(qr[c], k[c], s); dp = fmaf(gr[c], v[c], dp); }
-            float pr = 0.0f, ds = 0.0f;
-            const bool live = i < p.L && j < p.L && (!p.causal || j <= i) && lse > -CUDART_INF_F;
-            if (live) {
-                s *= p.scale;
-                if (bias) s += bias[static_cast<size_t>(i) * p.L + j];
-                pr = expf(s - lse);
-                ds = pr * (dp - Di);
-            }
-            dSw[lane * kRpw + r] = ds;
-            Pw[lane * kRpw + r] = pr;
-        }
-        __syncwarp();
-        // phase 2: lane = channel; dK[j][c] += dS[i][j] Q[i][c], dV[j][c] += P[i][j] dO[i][c] over the 32 queries
-#pragma unroll 4
-        for (int ii = 0; ii < kRows; ++ii) {
-            float dsr[kRpw], prr[kRpw];
-#pragma unroll
-            for (int r = 0; r < kRpw; ++r) { dsr[r] = dSw[ii * kRpw + r]; prr[r] = Pw[ii * kRpw + r]; }
-#pragma unroll
-            for (int a = 0; a < NACC; ++a) {
-                const int c = lane + 32 * a;
-                const float qv = (c < DP) ? Qs[ii * (DP + 1) + c] : 0.0f;
-                const float gv = (c < DP) ? dOs[ii * (DP + 1) + c] : 0.0f;
-#pragma unroll
-                for (int r = 0; r < kRpw; ++r) { ak[r][a] = fmaf(dsr[r], qv, ak[r][a]); av[r][a] = fmaf(prr[r], gv, av[r][a]); }
-            }
-        }
-        __syncwarp();
+        out.mac(probs, dOr, ov);
+        __syncthreads();
+        attn_store_probs<16>(probs, arow, bcol, s);
+        __syncthreads();
+        out.mac(probs, Qr, ok);
     }
-#pragma unroll
-    for (int r = 0; r < kRpw; ++r) {
-        const int j = j0 + warp * kRpw + r;
-#pragma unroll
-        for (int a = 0; a < NACC; ++a) {
-            const int c = lane + 32 * a;
-            if (j < p.L && c < p.d) {
-                if (p.dK) p.dK[base + static_cast<size_t>(j) * p.d + c] = p.scale * ak[r][a];
-                if (p.dV) p.dV[base + static_cast<size_t>(j) * p.d + c] = av[r][a];
-            }
-        }
+    if (p.dK) {
+        __syncthreads();
+        out.spill(probs, ok);
+        __syncthreads();
+        store_rows<DP>(p.dK + base, probs, j0, p.L, p.d, p.scale, p.vec_out);
+    }
+    if (p.dV) {
+        __syncthreads();
+        out.spill(probs, ov);
+        __syncthreads();
+        store_rows<DP>(p.dV + base, probs, j0, p.L, p.d, 1.0f, p.vec_out);
     }
 }
 
 template <int DP>
 int launch_dp(const BwdParams& p, cudaStream_t st) {
-    const dim3 grid((p.L + kRows - 1) / kRows, p.B * p.H);
+    const dim3 grid((p.L + kT - 1) / kT, p.B * p.H);
+    constexpr int dq_bytes = dq_smem_floats<DP>() * 4, dkv_bytes = dkv_smem_floats<DP>() * 4;
+    static bool configured[64] = {false};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) { cudaGetLastError(); return ST_LAUNCH; }
+    if (!configured[dev]) {
+        if (cudaFuncSetAttribute(attn_bwd_dq_kernel<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, dq_bytes) != cudaSuccess ||
+            cudaFuncSetAttribute(attn_bwd_dkv_kernel<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, dkv_bytes) != cudaSuccess) {
+            cudaGetLastError();
+            return ST_LAUNCH;
+        }
+        configured[dev] = true;
+    }
     if (p.dQ || p.dbias) {
-        const size_t smem = sizeof(float) * (2 * kRows * (DP + 1) + 2 * kRows * DP + kWarps * 32 * kRpw + 2 * kRows);
-        attn_bwd_dq_kernel<DP><<<grid, kWarps * 32, smem, st>>>(p);
+        attn_bwd_dq_kernel<DP><<<grid, kAttnThreads, dq_bytes, st>>>(p);
         if (cudaGetLastError() != cudaSuccess) return ST_LAUNCH;
     }
     if (p.dK || p.dV) {
-        const size_t smem = sizeof(float) * (2 * kRows * (DP + 1) + 2 * kRows * DP + 2 * kWarps * 32 * kRpw + 2 * kRows);
-        attn_bwd_dkv_kernel<DP><<<grid, kWarps * 32, smem, st>>>(p);
+        attn_bwd_dkv_kernel<DP><<<grid, kAttnThreads, dkv_bytes, st>>>(p);
         if (cudaGetLastError() != cudaSuccess) return ST_LAUNCH;
     }
     return ST_OK;
 }
+
+inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 }  // namespace
 
@@ -289,6 +340,10 @@ int launch_attn_backward(int B, int H, int L, int d, int causal, float scale, co
     p.B = B; p.H = H; p.L = L; p.d = d; p.causal = causal; p.scale = scale;
     p.Q = Q; p.K = K; p.V = V; p.bias = bias; p.O = O; p.dO = dO; p.LSE = LSE; p.bias_batch_stride = bias_batch_stride;
     p.dQ = dQ; p.dK = dK; p.dV = dV; p.dbias = dbias;
+    p.vec_in = d % 4 == 0 && aligned16(Q) && aligned16(K) && aligned16(V) && aligned16(O) && aligned16(dO);
+    p.vec_out = d % 4 == 0 && aligned16(dQ) && aligned16(dK) && aligned16(dV);
+    p.vec_bias = L % 4 == 0 && aligned16(bias) && bias_batch_stride % 4 == 0;
+    p.vec_dbias = L % 4 == 0 && aligned16(dbias);
     if (d <= 8) return launch_dp<8>(p, st);
     if (d <= 16) return launch_dp<16>(p, st);
     if (d <= 32) return launch_dp<32>(p, st);

@@ -592,6 +592,19 @@ def test_attention_backward(oracle, B, h, L, d, causal, bias, bcast, masked):
     assert torch.equal(part["dV"], got["dV"]) and torch.equal(part["dQ"], got["dQ"])
 
 
+@pytest.mark.parametrize("B,h,L,d,causal,bias", [(1, 2, 64, 32, False, True), (1, 2, 65, 32, True, True), (2, 1, 2, 32, False, True), (1, 1, 129, 64, True, True),
+                                                 (1, 2, 63, 3, False, True), (1, 2, 130, 10, True, False), (1, 1, 66, 61, False, True), (1, 3, 68, 16, False, True)])
+def test_attention_backward_tile_edges(oracle, B, h, L, d, causal, bias):
+    """Edges of the 64-row tiles and of the padded head dims, rows that are and are not whole 16-byte pieces; a fully masked row.  (Not one key alone: P = 1 there, dS = dP - D is 0 up to the rounding of two equal sums, and a
+    relative error of it has no bound.)"""
+    Q, K, V, bi, dO = cases.attn_backward_case(B, h, L, d, seed=21, bias=bias, masked_rows=(L - 1,) if bias else ())
+    O, LSE = oracle.flash_attn(Q, K, V, bi, scale=0.2, causal=causal)
+    ref = oracle.flash_attn_backward(Q, K, V, O, dO, LSE, bi, scale=0.2, causal=causal)
+    got = ops.flash_attn_backward_cuda(dev(Q), dev(K), dev(V), dev(O), dev(dO), dev(LSE), dev(bi) if bi is not None else None, scale=0.2, causal=causal)
+    for n in ("dQ", "dK", "dV", "dbias"):
+        assert cases.rel_err(host(got[n]), ref[n]) <= TOL_FP32, n
+
+
 def test_attention_backward_from_the_cuda_forward(oracle):
     """Forward on the tensor cores, backward on its O and LSE: the chain a training step runs (1e-3: the forward is tf32)."""
     Q, K, V, bi, dO = cases.attn_backward_case(2, 8, 128, 32, seed=9, bias_bcast=True)
