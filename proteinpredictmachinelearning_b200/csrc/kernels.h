@@ -79,6 +79,10 @@ int launch_attn_backward(int B, int H, int L, int d, int causal, float scale, co
 int launch_attn_d8_mma(const float* Q, const float* K, const float* V, const float* bias, float* O, float* LSE, int B, int H,
                        int L, int Lk, int d, int causal, float scale, float eps, long long bias_batch_stride, int ft,
                        const AttnLayout& lay, cudaStream_t st);
+// exact fp32, head dims 17 .. 64, sequences that fill 64 x 64 tiles (attn_exact.cu); ST_UNSUPPORTED_PATH otherwise
+int launch_attn_exact(const void* Q, const void* K, const void* V, int elem, const float* bias, float* O, float* LSE, int B, int H, int L,
+                      int Lk, int d, int causal, float scale, float eps, long long bias_batch_stride, int ft, const AttnLayout& lay,
+                      cudaStream_t st);
 int launch_attn_rowwarp(const void* Q, const void* K, const void* V, int elem, const float* bias, float* O, float* LSE,
                         int B, int H, int L, int Lk, int d, int causal, float scale, float eps,
                         long long bias_batch_stride, int ft, const AttnLayout& lay, cudaStream_t st);

@@ -1047,6 +1047,8 @@ int launch_attn_rowwarp(const void* Q, const void* K, const void* V, int elem, c
                                           bias, O, LSE, B, H, L, Lk, d, causal, scale, eps, bias_batch_stride, ft, lay, st);
         if (done) return cudaGetLastError() == cudaSuccess ? ST_OK : ST_LAUNCH;
     }
+    const int rx = launch_attn_exact(Q, K, V, elem, bias, O, LSE, B, H, L, Lk, d, causal, scale, eps, bias_batch_stride, ft, lay, st);
+    if (rx != ST_UNSUPPORTED_PATH) return rx;
     dim3 grid((L + 4 * kRowsPerWarp - 1) / (4 * kRowsPerWarp), H, B);
     const size_t smem = (32 * (d + 1) + 32 * d + 4 * kRowsPerWarp * (d + 32)) * sizeof(float);     // at most 43 KB (d = 128)
     auto go = [&](auto tag, auto dt) {

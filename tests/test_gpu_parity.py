@@ -592,6 +592,25 @@ def test_attention_backward(oracle, B, h, L, d, causal, bias, bcast, masked):
     assert torch.equal(part["dV"], got["dV"]) and torch.equal(part["dQ"], got["dQ"])
 
 
+@pytest.mark.parametrize("B,h,L,Lk,d,bias,causal,dtype", [
+    (1, 2, 64, 64, 32, True, False, None), (2, 2, 65, 129, 32, True, False, None), (1, 2, 127, 127, 32, False, True, None), (1, 3, 51, 51, 32, True, False, None),
+    (1, 2, 130, 70, 64, True, False, None), (1, 1, 96, 61, 41, True, False, None), (2, 1, 100, 90, 20, True, False, torch.bfloat16),
+    (2, 2, 70, 70, 32, True, False, None), (1, 2, 33, 300, 64, False, False, torch.float16)])
+def test_attention_exact_tile_edges(oracle, B, h, L, Lk, d, bias, causal, dtype):
+    """The exact kernel for head dims 17 .. 64 at the edges of its 64 x 64 tiles and of its rule (70 x 70 goes to the 16-row kernel),
+    rows that are and are not whole groups of four, a fully masked row and one whose first key tile is masked."""
+    Q, K, V, bi = cases.attn_case(B, h, L, d, Lk=Lk, seed=22, bias=bias)
+    if bias:
+        bi[:, :, 5, :] = -np.inf
+        bi[:, :, 7, :64] = -np.inf
+    t = [dev(x) if dtype is None else dev(x, dtype) for x in (Q, K, V)]
+    O, LSE = ops.flash_attn_forward_cuda(*t, dev(bi) if bias else None, scale=0.2, causal=causal, path=PATH_SIMT)
+    rO, rL = oracle.flash_attn(*[host(x.float()) for x in t], bi, scale=0.2, causal=causal)
+    assert cases.rel_err(host(O), rO) <= TOL_FP32
+    fin = np.isfinite(rL)
+    assert np.array_equal(np.isfinite(host(LSE)), fin) and np.abs(host(LSE)[fin] - rL[fin]).max() <= 1e-5
+
+
 @pytest.mark.parametrize("B,h,L,d,causal,bias", [(1, 2, 64, 32, False, True), (1, 2, 65, 32, True, True), (2, 1, 2, 32, False, True), (1, 1, 129, 64, True, True),
                                                  (1, 2, 63, 3, False, True), (1, 2, 130, 10, True, False), (1, 1, 66, 61, False, True), (1, 3, 68, 16, False, True)])
 def test_attention_backward_tile_edges(oracle, B, h, L, d, causal, bias):
