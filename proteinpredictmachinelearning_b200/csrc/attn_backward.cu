@@ -12,9 +12,12 @@
 // the same buffer) to shared memory as [partner][own row], then the result's register tile over the partners (attn_tile.cuh).
 //
 // Bound: instruction issue (fp32 FMAs are half of it: 3 products in one kernel, 4 in the other; FMA pipe 45 % busy at two CTAs
-// per SM).  64 x 8 x 256 x 32 with dbias 1535 -> 510 us (30 TFLOP/s over the seven products), head dim 8 613 -> 259 us, against the form with a warp per 8 rows, whose lanes read one scalar from shared memory per FMA or two.  The next
-// tile and this tile's bias are requested before the products (255 registers, two CTAs per SM): 573 us with three CTAs per SM
-// that wait for them.
+// per SM).  64 x 8 x 256 x 32 with dbias 1535 -> 510 us (30 TFLOP/s over the seven products), head dim 8 613 -> 259 us, against
+// 32-row tiles with a warp per 8 rows, whose lanes read one scalar from shared memory per FMA or two.  The next tile and this
+// tile's bias are requested before the products (255 registers, two CTAs per SM): 573 us with three CTAs per SM that wait for
+// them.  Sequences that fit one tile of 32 rows keep that form (attn_backward_short.cu, with both sides' times); above, the
+// 64-row tiles are faster throughout, also where they are emptiest (256 x 8, 33 rows: 120 -> 76, 343 -> 142 and 641 -> 255 us for
+// head dims 8, 32 and 64; 72 rows: 279 -> 257, 801 -> 510, 1434 -> 916).
 // Layouts as the forward: Q, K, V, O, dO, dQ, dK, dV [B, h, L, d]; bias [B, h, L, L] with a batch stride (0: shared);
 // dbias [B, h, L, L]; LSE [B, h, L].  d <= 64.
 #include <cuda_runtime.h>
@@ -336,6 +339,8 @@ int launch_attn_backward(int B, int H, int L, int d, int causal, float scale, co
                          const float* bias, long long bias_batch_stride, const float* O, const float* dO, const float* LSE,
                          float* dQ, float* dK, float* dV, float* dbias, cudaStream_t st) {
     if (d > 64 || static_cast<long long>(B) * H > 65535) return ST_UNSUPPORTED_PATH;
+    if (L <= kAttnBackwardShortRows)
+        return launch_attn_backward_short(B, H, L, d, causal, scale, Q, K, V, bias, bias_batch_stride, O, dO, LSE, dQ, dK, dV, dbias, st);
     BwdParams p;
     p.B = B; p.H = H; p.L = L; p.d = d; p.causal = causal; p.scale = scale;
     p.Q = Q; p.K = K; p.V = V; p.bias = bias; p.O = O; p.dO = dO; p.LSE = LSE; p.bias_batch_stride = bias_batch_stride;

@@ -624,6 +624,28 @@ def test_attention_backward_tile_edges(oracle, B, h, L, d, causal, bias):
         assert cases.rel_err(host(got[n]), ref[n]) <= TOL_FP32, n
 
 
+@pytest.mark.parametrize("B,h,L,d,causal,bias", [(1, 2, 32, 32, False, True), (1, 2, 31, 32, True, True), (3, 8, 8, 32, False, True), (2, 1, 2, 64, False, False),
+                                                 (1, 2, 33, 64, True, True), (1, 2, 17, 3, False, True), (2, 2, 32, 8, True, False), (1, 1, 9, 61, True, True)])
+def test_attention_backward_short(oracle, B, h, L, d, causal, bias):
+    """Sequences of at most 32 rows (one tile per batch and head) and the first longer one; a fully masked row; only some gradients
+    wanted.  The bias and its gradient start 4 bytes off a 16-byte boundary."""
+    Q, K, V, bi, dO = cases.attn_backward_case(B, h, L, d, seed=23, bias=bias, masked_rows=(L - 1,) if bias else ())
+    O, LSE = oracle.flash_attn(Q, K, V, bi, scale=0.2, causal=causal)
+    ref = oracle.flash_attn_backward(Q, K, V, O, dO, LSE, bi, scale=0.2, causal=causal)
+    shifted = lambda shape: torch.zeros(int(np.prod(shape)) + 1, device="cuda")[1:].view(*shape)
+    db = None
+    if bi is not None:
+        db = shifted(bi.shape)
+        db.copy_(dev(bi))
+    got = {n: shifted(ref[n].shape) for n in ("dQ", "dK", "dV", "dbias")}
+    args = [dev(x) for x in (Q, K, V, O, dO, LSE)]
+    ops.flash_attn_backward_cuda(*args, db, scale=0.2, causal=causal, out=got)
+    for n in got:
+        assert cases.rel_err(host(got[n]), ref[n]) <= TOL_FP32, n
+    for n in got:
+        assert torch.equal(ops.flash_attn_backward_cuda(*args, db, scale=0.2, causal=causal, want=(n,))[n], got[n]), n
+
+
 def test_attention_backward_from_the_cuda_forward(oracle):
     """Forward on the tensor cores, backward on its O and LSE: the chain a training step runs (1e-3: the forward is tf32)."""
     Q, K, V, bi, dO = cases.attn_backward_case(2, 8, 128, 32, seed=9, bias_bcast=True)
