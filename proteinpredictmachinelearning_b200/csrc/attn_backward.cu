@@ -9,7 +9,8 @@
 //   attn_bwd_dq_kernel   one CTA = 64 query rows of one (batch, head); walks the key tiles of 64; writes dQ and dbias
 //   attn_bwd_dkv_kernel  one CTA = 64 key rows of one (batch, head); walks the query tiles of 64; writes dK and dV
 // Per tile: scores and dP as register tiles over the channels, exp and dS in registers, dS (and P, one after the other through
-// the same buffer) to shared memory as [partner][own row], then the result's register tile over the partners (attn_tile.cuh).
+// the same buffer) to shared memory as [partner][own row], then the result's register tile over the partners (attn_tile.cuh).  A causal row takes
+// nothing from the partner rows beyond its diagonal, whatever values they hold.
 //
 // Bound: instruction issue (fp32 FMAs are half of it: 3 products in one kernel, 4 in the other; FMA pipe 45 % busy at two CTAs
 // per SM).  64 x 8 x 256 x 32 with dbias 1535 -> 510 us (30 TFLOP/s over the seven products), head dim 8 613 -> 259 us, against
@@ -176,7 +177,8 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_bwd_dq_kernel(const BwdP
         if (p.dQ) {
             attn_store_probs<16>(probs, arow, bcol, s);
             __syncthreads();
-            out.mac(probs, Kr, o);
+            if (p.causal && j0 == i0) out.template mac_diag<false>(probs, Kr, o);
+            else out.mac(probs, Kr, o);
         }
     }
     // keys past jend of a causal CTA: dbias stays 0 there
@@ -285,11 +287,14 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_bwd_dkv_kernel(const Bwd
 #pragma unroll
             for (int u = 0; u < 4; ++u) s[r][u] = (r < 4 ? r : 12 + r) < keys[u] ? s[r][u] * (dp[r][u] - Di[u]) : 0.0f;
         __syncthreads();
-        out.mac(probs, dOr, ov);
+        const bool diag = p.causal && i0 == j0;
+        if (diag) out.template mac_diag<true>(probs, dOr, ov);
+        else out.mac(probs, dOr, ov);
         __syncthreads();
         attn_store_probs<16>(probs, arow, bcol, s);
         __syncthreads();
-        out.mac(probs, Qr, ok);
+        if (diag) out.template mac_diag<true>(probs, Qr, ok);
+        else out.mac(probs, Qr, ok);
     }
     if (p.dK) {
         __syncthreads();

@@ -128,7 +128,8 @@ attn_exact_kernel(const T* __restrict__ Q, const T* __restrict__ K, const T* __r
 #pragma unroll
                 for (int c = 0; c < NC; ++c) o[i][c] *= a[i];
         }
-        out.mac(probs, Vr, o);
+        if (p.causal && j0 == i0) out.template mac_diag<false>(probs, Vr, o);
+        else out.mac(probs, Vr, o);
     }
 
     __syncthreads();                                  // probs and rowf are no longer read

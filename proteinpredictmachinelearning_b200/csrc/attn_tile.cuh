@@ -99,7 +99,7 @@ __device__ __forceinline__ void attn_scores(const float* at, const float* bt, in
 }
 
 // Where a thread's part of the result [64][DP] lies.  Narrow results would leave a thread too few outputs per shared-memory read,
-// so the partners of a tile are shared among kGroups groups of warps, each with the whole result; attn_reduce adds them.
+// so the partners of a tile are shared among kGroups groups of warps, each with the whole result; sum() adds them.
 template <int DP>
 struct AttnOut {
     static constexpr int kCols = DP >= 16 ? 4 : 2;                               // columns per thread (rows: 8)
@@ -141,6 +141,27 @@ struct AttnOut {
 #pragma unroll
                     for (int i = 0; i < 8; i += 2)
                         unpack2(ffma2(pack2(a[i], a[i + 1]), b2, pack2(o[i][c], o[i + 1][c])), o[i][c], o[i + 1][c]);
+                }
+            }
+        }
+    }
+    // The same for the tile on the diagonal of a causal attention: a partner enters only the rows that see it (partner <= row, or
+    // with OWN_IS_KEY partner >= row).  Their probability is zero as well, but zero times an infinity or a NaN in a partner row is not.
+    template <bool OWN_IS_KEY>
+    __device__ __forceinline__ void mac_diag(const float* probs, const float* rm, float (&o)[8][kCols]) const {
+#pragma unroll 1
+        for (int j = group * kPartners; j < (group + 1) * kPartners; ++j) {
+            const int sw = attn_swz_p(j);
+            float a[8];
+            *reinterpret_cast<float4*>(a) = *reinterpret_cast<const float4*>(probs + j * kAttnTile + (row ^ sw));
+            *reinterpret_cast<float4*>(a + 4) = *reinterpret_cast<const float4*>(probs + j * kAttnTile + ((row + kStep) ^ sw));
+#pragma unroll
+            for (int c = 0; c < kCols; ++c) {
+                const float b = rm[j * DP + col + c];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const int r = row + (i < 4 ? i : kStep - 4 + i);
+                    if (OWN_IS_KEY ? j >= r : j <= r) o[i][c] = fmaf(a[i], b, o[i][c]);
                 }
             }
         }

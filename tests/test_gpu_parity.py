@@ -646,6 +646,41 @@ def test_attention_backward_short(oracle, B, h, L, d, causal, bias):
         assert torch.equal(ops.flash_attn_backward_cuda(*args, db, scale=0.2, causal=causal, want=(n,))[n], got[n]), n
 
 
+@pytest.mark.parametrize("d,dtype", [(32, None), (64, None), (20, None), (32, torch.bfloat16)])
+def test_attention_exact_causal_ignores_what_a_row_does_not_see(d, dtype):
+    """Infinities and NaNs in V of later keys of the same tile: the rows before them keep their bits."""
+    Q, K, V, _ = cases.attn_case(1, 2, 130, d, seed=24, bias=False)
+    t = [dev(x) if dtype is None else dev(x, dtype) for x in (Q, K, V)]
+    ref = ops.flash_attn_forward_cuda(*t, None, scale=0.2, causal=True, path=PATH_SIMT)[0]
+    for j, value in ((70, np.inf), (63, np.nan), (129, -np.inf)):
+        bad = t[2].clone()
+        bad[:, :, j] = value
+        got = ops.flash_attn_forward_cuda(t[0], t[1], bad, None, scale=0.2, causal=True, path=PATH_SIMT)[0]
+        assert torch.equal(got[:, :, :j], ref[:, :, :j]) and not torch.isfinite(got[:, :, j:]).any(), j
+
+
+@pytest.mark.parametrize("d", [8, 16, 32, 64])
+def test_attention_backward_causal_ignores_what_a_row_does_not_see(d):
+    """The same for the gradients: a bad key row reaches the queries from it on, a bad query row the keys up to it."""
+    Q, K, V, _, dO = cases.attn_backward_case(1, 2, 130, d, seed=25, bias=False)
+    q, k, v, do = (dev(x) for x in (Q, K, V, dO))
+    o, lse = ops.flash_attn_forward_cuda(q, k, v, None, scale=0.2, causal=True, path=PATH_SIMT)
+    grads = lambda q, k, v, do: ops.flash_attn_backward_cuda(q, k, v, o, do, lse, None, scale=0.2, causal=True)
+    ref = grads(q, k, v, do)
+    for j, value in ((70, np.inf), (63, np.nan), (20, -np.inf)):
+        bk, bv, bq, bdo = k.clone(), v.clone(), q.clone(), do.clone()
+        for x in (bk, bv, bq, bdo):
+            x[:, :, j] = value
+        got = grads(q, bk, bv, do)
+        assert torch.equal(got["dQ"][:, :, :j], ref["dQ"][:, :, :j]), j
+        for n in ("dK", "dV"):
+            assert torch.equal(got[n][:, :, :j], ref[n][:, :, :j]) and torch.equal(got[n][:, :, j + 1:], ref[n][:, :, j + 1:]), (j, n)
+        got = grads(bq, k, v, bdo)
+        for n in ("dK", "dV"):
+            assert torch.equal(got[n][:, :, j + 1:], ref[n][:, :, j + 1:]), (j, n)
+        assert torch.equal(got["dQ"][:, :, :j], ref["dQ"][:, :, :j]) and torch.equal(got["dQ"][:, :, j + 1:], ref["dQ"][:, :, j + 1:]), j
+
+
 def test_attention_backward_from_the_cuda_forward(oracle):
     """Forward on the tensor cores, backward on its O and LSE: the chain a training step runs (1e-3: the forward is tf32)."""
     Q, K, V, bi, dO = cases.attn_backward_case(2, 8, 128, 32, seed=9, bias_bcast=True)
