@@ -237,6 +237,29 @@ def cpu_baseline_record(budget_s=10.0):
             "sample": f"{CPU_SAMPLE_NOTE}; {reps} pass(es)"}
 
 
+# records beside the contract keys: a line with all of them is some 25 KB, more than a reader that keeps the end of the output sees
+DETAIL_KEYS = ("per_shape", "kernels", "dev_forward_calls", "sharded_block", "sharded_extra_block", "reference_cpu_kernels")
+
+
+def print_line(line):
+    """One JSON line on stdout with the contract keys and the detail records' headline figures; the records themselves on
+    stderr, one JSON line each."""
+    line = dict(line)
+    brief = {}
+    for key in DETAIL_KEYS:
+        rec = line.pop(key, None)
+        if rec is None:
+            continue
+        print(json.dumps({"detail": key, "record": rec}), file=sys.stderr, flush=True)
+        if isinstance(rec, dict):
+            brief[key] = {k: rec[k] for k in ("ms_per_block", "us_per_forward_hot_path", "calls_checked", "worst_err", "checked") if k in rec}
+        else:
+            brief[key] = len(rec)
+    if brief:
+        line["detail_on_stderr"] = brief
+    print(json.dumps(line), flush=True)
+
+
 def run_reference(args):
     rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
@@ -263,7 +286,7 @@ def run_reference(args):
     }
     if not args.no_kernels:
         line["reference_cpu_kernels"] = reference_cpu_kernels()
-    print(json.dumps(line), flush=True)
+    print_line(line)
 
 
 # ------------------------------------------------------------------------------------------------
@@ -769,8 +792,8 @@ def run_ours(args):
     if world == 1 and not args.no_cpu_baseline:
         line["cpu_baseline"] = cpu_baseline_record()
         if not args.no_kernels:
-            line["cpu_baseline"]["reference_cpu_kernels"] = reference_cpu_kernels()
-    print(json.dumps(line), flush=True)
+            line["reference_cpu_kernels"] = reference_cpu_kernels()
+    print_line(line)
     if world > 1:
         dist.destroy_process_group()
 
