@@ -147,6 +147,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_bwd_dq_kernel(const BwdP
         __syncthreads();                               // the tiles of the previous step are no longer read
         rk.template store<true, true>(Kt, Kr);
         rv.template store<true, false>(Vt, nullptr);
+        const bool diag = p.causal && j0 == i0, fin = !diag || rk.finite();
         const int j = j0 + bcol;
         float4 bi[8];                                  // this tile's bias and the next tile's keys travel during the products
 #pragma unroll
@@ -158,7 +159,9 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_bwd_dq_kernel(const BwdP
             rk.fetch(p.K + base, p.d, j0 + kT, p.L, p.d, p.vec_in);
             rv.fetch(p.V + base, p.d, j0 + kT, p.L, p.d, p.vec_in);
         }
-        __syncthreads();
+        bool masked = false;                           // unseen K rows may not even be multiplied by zero
+        if (diag) masked = __syncthreads_or(!fin);
+        else __syncthreads();
         float s[8][4], dp[8][4];
         attn_scores<DP, 16>(Qt, Kt, arow, bcol, s);
         attn_scores<DP, 16>(dOt, Vt, arow, bcol, dp);
@@ -177,7 +180,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_bwd_dq_kernel(const BwdP
         if (p.dQ) {
             attn_store_probs<16>(probs, arow, bcol, s);
             __syncthreads();
-            if (p.causal && j0 == i0) out.template mac_diag<false>(probs, Kr, o);
+            if (masked) out.template mac_diag<false>(probs, Kr, o);
             else out.mac(probs, Kr, o);
         }
     }
@@ -250,6 +253,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_bwd_dkv_kernel(const Bwd
         rg.template store<true, true>(dOt, dOr);
         store_row_dots<DP>(rg, ro, Dr);
         if (threadIdx.x < kT) Ls[threadIdx.x] = rl;
+        const bool diag = p.causal && i0 == j0, fin = !diag || (rq.finite() && rg.finite());
         float4 bi[4][2];                               // this tile's bias and the next query tile travel during the products
 #pragma unroll
         for (int u = 0; u < 4; ++u)
@@ -260,7 +264,9 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_bwd_dkv_kernel(const Bwd
                                                : make_float4(0.f, 0.f, 0.f, 0.f);
             }
         if (i0 + kT < p.L) fetch_queries(i0 + kT);
-        __syncthreads();
+        bool masked = false;                           // Q and dO rows that do not see a key may not even be multiplied by zero
+        if (diag) masked = __syncthreads_or(!fin);
+        else __syncthreads();
         float s[8][4], dp[8][4];
         attn_scores<DP, 16>(Kt, Qt, arow, bcol, s);    // [key][query]
         const float4 l4 = attn_ld4(Ls + bcol);
@@ -287,13 +293,12 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_bwd_dkv_kernel(const Bwd
 #pragma unroll
             for (int u = 0; u < 4; ++u) s[r][u] = (r < 4 ? r : 12 + r) < keys[u] ? s[r][u] * (dp[r][u] - Di[u]) : 0.0f;
         __syncthreads();
-        const bool diag = p.causal && i0 == j0;
-        if (diag) out.template mac_diag<true>(probs, dOr, ov);
+        if (masked) out.template mac_diag<true>(probs, dOr, ov);
         else out.mac(probs, dOr, ov);
         __syncthreads();
         attn_store_probs<16>(probs, arow, bcol, s);
         __syncthreads();
-        if (diag) out.template mac_diag<true>(probs, Qr, ok);
+        if (masked) out.template mac_diag<true>(probs, Qr, ok);
         else out.mac(probs, Qr, ok);
     }
     if (p.dK) {

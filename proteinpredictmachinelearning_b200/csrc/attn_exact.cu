@@ -72,11 +72,14 @@ attn_exact_kernel(const T* __restrict__ Q, const T* __restrict__ K, const T* __r
         __syncthreads();                              // the tiles of the previous step are no longer read
         rk.template store<true, false>(Kt, nullptr);
         rv.template store<false, true>(nullptr, Vr);
+        const bool diag = p.causal && j0 == i0, fin = !diag || rv.finite();
         if (j0 + kT < jend) {
             rk.fetch(Kb, lay.k_l, j0 + kT, p.Lk, p.d, p.vec_k);
             rv.fetch(Vb, lay.v_l, j0 + kT, p.Lk, p.d, p.vec_v);
         }
-        __syncthreads();
+        bool masked = false;                          // unseen V rows may not even be multiplied by zero
+        if (diag) masked = __syncthreads_or(!fin);
+        else __syncthreads();
         float s[8][4];
         attn_scores<DP, 8>(Qt, Kt, arow, bcol, s);
         const int j = j0 + bcol;
@@ -128,7 +131,7 @@ attn_exact_kernel(const T* __restrict__ Q, const T* __restrict__ K, const T* __r
 #pragma unroll
                 for (int c = 0; c < NC; ++c) o[i][c] *= a[i];
         }
-        if (p.causal && j0 == i0) out.template mac_diag<false>(probs, Vr, o);
+        if (masked) out.template mac_diag<false>(probs, Vr, o);
         else out.mac(probs, Vr, o);
     }
 

@@ -59,6 +59,13 @@ struct AttnRows {
             }
         }
     }
+    // no infinity and no NaN among this thread's values
+    __device__ __forceinline__ bool finite() const {
+        float t = 0.0f;
+#pragma unroll
+        for (int it = 0; it < kN; ++it) t = fmaf(v[it].x, 0.0f, fmaf(v[it].y, 0.0f, fmaf(v[it].z, 0.0f, fmaf(v[it].w, 0.0f, t))));
+        return t == 0.0f;
+    }
     template <bool TR, bool RM>
     __device__ __forceinline__ void store(float* tr, float* rm) const {
         const int c = chan();
@@ -145,8 +152,10 @@ struct AttnOut {
             }
         }
     }
-    // The same for the tile on the diagonal of a causal attention: a partner enters only the rows that see it (partner <= row, or
-    // with OWN_IS_KEY partner >= row).  Their probability is zero as well, but zero times an infinity or a NaN in a partner row is not.
+    // The same for a tile on the diagonal of a causal attention whose partner rows hold an infinity or a NaN: a partner enters only the
+    // rows that see it (partner <= row, or with OWN_IS_KEY partner >= row).  For the others its probability is zero, which is enough
+    // for finite values (the kernels ask while they store the tile; this form on every diagonal tile made 51 x 8 x 51 x 32 causal 48 us
+    // instead of 40 backward).
     template <bool OWN_IS_KEY>
     __device__ __forceinline__ void mac_diag(const float* probs, const float* rm, float (&o)[8][kCols]) const {
 #pragma unroll 1
