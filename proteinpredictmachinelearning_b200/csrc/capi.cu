@@ -393,7 +393,7 @@ int ppml_b200_out_prod(const float* src0, const float* src1, float* dst,
     p.a_s2 = ne00 * ne01; p.a_s3 = ne00 * ne01 * ne02; p.a_div2 = ne2 / ne02; p.a_div3 = ne3 / ne03;
     p.b_s2 = ne10 * ne11; p.b_s3 = ne10 * ne11 * ne12;
     p.c_s2 = ne0 * ne1; p.c_s3 = ne0 * ne1 * ne2;
-    p.alpha = 1.0f; p.may_split = 1;
+    p.alpha = 1.0f;
     return launch_simt_contract(src0, src1, dst, p, 0, as_stream(stream));
 }
 

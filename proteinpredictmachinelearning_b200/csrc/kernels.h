@@ -19,7 +19,6 @@ struct SimtContract {
     long long a_s2, a_s3, a_div2, a_div3;
     long long b_s2, b_s3, c_s2, c_s3;
     long long b_div2, b_div3;   // 0 = 1
-    int may_split;              // 1: the contraction may be split over CTAs (changes the summation order)
     int vec_c;                  // set by the launcher: 16-byte stores are legal
     const float* bias;
     int bias_seed;              // 1: accumulator starts at bias[n] (fp32 mul_mat); 0: added at the end
@@ -106,7 +105,7 @@ struct UmmaGemmArgs {
     int tf32_mode;                     // fp32 only: 0 round in smem (rna), 1 TMA tf32 type, 2 truncate
     int mn_major;                      // 1: A[b][k][m], B[b][k][n] (row index contiguous; lda / ldb = k pitch), fp32 only
     const float* ln_stats; const float* ln_u; const float* gate; int act;      // fused LayerNorm algebra / activation gate
-    int may_split;                     // 1: the contraction may be split over CTAs (mn_major, fp32; no bias, no clamp)
+    int may_split;                     // 1: the contraction may be computed in parts (mn_major, fp32; no bias, no clamp)
 };
 int launch_umma_gemm(const UmmaGemmArgs& a, cudaStream_t st);
 

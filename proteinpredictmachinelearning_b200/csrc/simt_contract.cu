@@ -3,17 +3,16 @@
 //
 //   D[p][m][n] = epi( sum_k A[pa][m][k] * B[pb][n][k] )
 //
-// Each output element is one chain of fused multiply-adds with k ascending, the reference's order (unless the contraction is
-// split, see below), so fp32 results agree with its CPU kernels to rounding.
+// Each output element is one chain of fused multiply-adds with k ascending, the reference's order, so fp32 results agree with
+// its CPU kernels to rounding and do not depend on which of the kernels below, or how many planes, a call runs.
 #include "kernels.h"
 
-#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
-#include <mutex>
+#include <type_traits>
 
-namespace cg = cooperative_groups;
+#include "common.cuh"
 
 namespace ppml_b200 {
 
@@ -276,86 +275,112 @@ simt_contract_kernel(const T* __restrict__ A, const T* __restrict__ B, float* __
     }
 }
 
-// The split form, for plain products whose contraction is long and whose result is small (weight gradients: K = the tokens):
-// a CTA is two or four groups of four warps, a cluster up to 16 CTAs, and the groups take the slices of k of one 64 x 64 tile in turn, with
-// stages and a barrier of their own.  The partial tiles are left in shared memory and added piece by piece over the cluster in
-// the order of the groups (no atomics: the result does not depend on timing).
+// The narrow form, for plain fp32 products with the row index contiguous in both operands, a long contraction and a small result
+// (weight gradients: K = the tokens).  64 x 64 tiles would occupy a handful of SMs, and the contraction itself is not split: every
+// output stays one ascending chain.  So the tiles are 32 x 16, two warps with 4 x 2 outputs per thread, and three slices are on
+// their way through cp.async.
 //
-// Bound: FMA issue with 16 or more tiles; latency of a group's loads below that (one slice in flight per group), which is why
-// the ways are many and short.  256 x 256 over 65536 tokens 4850 -> 289 us (one CTA per 64 x 64 tile before), 64 x 256 over
-// 30000 1490 -> 63 us, 33 x 32 over 30000 1470 -> 76 us.  A group's slices lie next to the other groups', not in a range of its
-// own: all of them then move through the operands together.
-template <typename T, Fetch F, int kSplitGroups>
-__global__ void __launch_bounds__(kSplitGroups * 128, 4 / kSplitGroups)
-simt_contract_split_kernel(const T* __restrict__ A, const T* __restrict__ B, float* __restrict__ C, const SimtContract p, int n_tiles) {
-    constexpr int BM = 64, BN = 64;
-    static_assert(BM * BN == 2 * kSlice * (BM + BN), "a partial tile fills its group's stages");
-    extern __shared__ __align__(16) float dyn[];
-    cg::cluster_group cl = cg::this_cluster();
-    const int splits = static_cast<int>(cl.num_blocks()), rank = static_cast<int>(cl.block_rank());
-    const int grp = threadIdx.x >> 7, gtid = threadIdx.x & 127;
-    float* const As = dyn + grp * (BM * BN);
-    float* const Bs = As + 2 * kSlice * BM;
-    const int warp = gtid >> 5, lane = gtid & 31;
-    const int arow = (warp >> 1) * 32 + lane_m(lane) * 4, bcol = (warp & 1) * 32 + lane_n(lane) * 4;
+// Bound: with a CTA per SM the issue of its two warps and the restart after each slice's barrier (16 cycles per k: 10 instructions, of which 8
+// FMAs); with several, shared-memory reads (24 bytes per thread and k: 12 cycles per k and CTA, broadcast or not).  128 x 256 over
+// 2601 tokens 135 -> 24 us, 256 x 256 over 65536 4793 -> 553, 64 x 64 over 65536 3214 -> 526 (64 x 64 tiles of 256 threads before).
+// 2 x 2 outputs per thread on four warps with slices of 32: 28 us and 640; one warp with a 16 x 16 tile: 26 and 613.
+// Dealing the slices to the groups of a cluster and adding the partial sums took 16 and 273 us and came closer to the 64-bit result
+// (1.9e-7 against 9.1e-7 at 2601 tokens), but it is not the order that the callers of this path are promised, and the sum
+// depended on the number of planes.
+constexpr int kNarrowSlice = 64, kNarrowDepth = 4, kNarrowM = 32, kNarrowN = 16, kNarrowThreads = 64;
+
+__device__ __forceinline__ void cp_async(uint32_t dst, const float* src, bool in, std::integral_constant<int, 16>) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(in ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async(uint32_t dst, const float* src, bool in, std::integral_constant<int, 4>) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(in ? 4 : 0) : "memory");
+}
+
+// A thread's copies of one operand [k][row] into the stages [kNarrowSlice][ROWS], VEC elements each, slice after slice; zeros outside
+// the operand.
+template <int ROWS, int VEC>
+struct NarrowCopy {
+    static constexpr int kPerRow = ROWS / VEC, kRound = kNarrowThreads / kPerRow;        // copies per k; k per round of the CTA
+    static_assert(kNarrowThreads % kPerRow == 0 && kNarrowSlice % kRound == 0, "whole k per round");
+    const float* ptr;
+    const float* base;
+    long long delta;
+    int k, dst;
+    bool in;
+    __device__ __forceinline__ void init(const float* src, long long s_k, int rows_left) {
+        const int r = (static_cast<int>(threadIdx.x) % kPerRow) * VEC;
+        k = static_cast<int>(threadIdx.x) / kPerRow;
+        in = r < rows_left;
+        base = src;
+        ptr = in ? src + k * s_k + r : src;
+        delta = kRound * s_k;
+        dst = k * ROWS + r;
+    }
+    __device__ __forceinline__ void fetch(float* stage, int k_left) {
+        const uint32_t d = smem_u32(stage + dst);
+#pragma unroll
+        for (int i = 0; i < kNarrowSlice / kRound; ++i) {
+            const bool ok = in && k + i * kRound < k_left;
+            cp_async(d + i * kRound * ROWS * 4, ok ? ptr + i * delta : base, ok, std::integral_constant<int, 4 * VEC>());
+        }
+        ptr += in ? (kNarrowSlice / kRound) * delta : 0;
+    }
+};
+
+template <int VEC>
+__global__ void __launch_bounds__(kNarrowThreads, 4)
+simt_contract_narrow_kernel(const float* __restrict__ A, const float* __restrict__ B, float* __restrict__ C, const SimtContract p, int n_tiles) {
+    constexpr int BM = kNarrowM, BN = kNarrowN, kStage = kNarrowSlice * (BM + BN), kDepth = kNarrowDepth;
+    __shared__ __align__(16) float stages[kDepth * kStage];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int arow = warp * 16 + (lane & 3) * 4, bcol = (lane >> 2) * 2;
     const int mt = blockIdx.x / n_tiles;
     const long long m0 = static_cast<long long>(mt) * BM, n0 = static_cast<long long>(blockIdx.x - mt * n_tiles) * BN;
-    const PlanePtrs<T> pp = plane_ptrs(A, B, C, p, blockIdx.z / splits);
+    const int a_left = static_cast<int>(min(p.M - m0, static_cast<long long>(BM))), b_left = static_cast<int>(min(p.N - n0, static_cast<long long>(BN)));
+    const int slices = static_cast<int>((p.K + kNarrowSlice - 1) / kNarrowSlice);
 
-    const long long ways = static_cast<long long>(splits) * kSplitGroups;
-    const long long kbeg = (rank * kSplitGroups + grp) * static_cast<long long>(kSlice), kstep = ways * kSlice;
-    long long k_left = p.K - kbeg;                       // not positive: a group without a share
-    float acc[8][4];
+    for (long long plane = blockIdx.z; plane < p.planes; plane += gridDim.z) {
+        const PlanePtrs<float> pp = plane_ptrs(A, B, C, p, plane);
+        NarrowCopy<BM, VEC> ca;
+        NarrowCopy<BN, VEC> cb;
+        ca.init(pp.a + m0, p.a_sk, a_left);
+        cb.init(pp.b + n0, p.b_sk, b_left);
+        auto fetch = [&](int s) {
+            if (s < slices) {
+                float* st = stages + (s % kDepth) * kStage;
+                const int k_left = static_cast<int>(min(p.K - static_cast<long long>(s) * kNarrowSlice, static_cast<long long>(kNarrowSlice)));
+                ca.fetch(st, k_left);
+                cb.fetch(st + kNarrowSlice * BM, k_left);
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        float acc[4][2];
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
+        for (int i = 0; i < 4; ++i) { acc[i][0] = 0.0f; acc[i][1] = 0.0f; }
+        __syncthreads();                                 // the stages of the previous plane are no longer read
+        for (int s = 0; s < kDepth - 1; ++s) fetch(s);
+        for (int s = 0; s < slices; ++s) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(kDepth - 2) : "memory");
+            __syncthreads();                             // slice s has arrived for everyone, slice s - 1 is no longer read
+            fetch(s + kDepth - 1);
+            const float* as = stages + (s % kDepth) * kStage + arow;
+            const float* bs = stages + (s % kDepth) * kStage + kNarrowSlice * BM + bcol;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
-    auto group_sync = [&] { asm volatile("bar.sync %0, 128;" ::"r"(grp + 1) : "memory"); };
-    Loader<T, F, BM, 128> la;
-    Loader<T, F, BN, 128> lb;
-    la.init(pp.a, gtid, m0, p.M, kbeg, p.a_sm, p.a_sk, ways);
-    lb.init(pp.b, gtid, n0, p.N, kbeg, p.b_sn, p.b_sk, ways);
-    la.fetch(gtid, clip_slice(k_left));
-    lb.fetch(gtid, clip_slice(k_left));
-    la.store(gtid, As);
-    lb.store(gtid, Bs);
-    group_sync();
-    int buf = 0;
-    for (; k_left > 0; k_left -= kstep, buf ^= 1) {
-        const bool more = k_left > kstep;
-        if (more) {
-            la.fetch(gtid, clip_slice(k_left - kstep));
-            lb.fetch(gtid, clip_slice(k_left - kstep));
-        }
-        mac_slice<F, BM, BN, 4>(As + buf * (kSlice * BM), Bs + buf * (kSlice * BN), arow, bcol, acc);
-        if (more) {
-            la.store(gtid, As + (buf ^ 1) * (kSlice * BM));
-            lb.store(gtid, Bs + (buf ^ 1) * (kSlice * BN));
-        }
-        group_sync();
-    }
+            for (int kk = 0; kk < kNarrowSlice; ++kk) {
+                float a[4];
+                *reinterpret_cast<float4*>(a) = load4(as + kk * BM);
+                const float2 b = *reinterpret_cast<const float2*>(bs + kk * BN);
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
-        *reinterpret_cast<float4*>(As + (arow + (i < 4 ? i : 12 + i)) * BN + bcol) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
-    cl.sync();
-    for (int e = rank * (kSplitGroups * 128) + static_cast<int>(threadIdx.x); e < BM * BN / 4; e += splits * (kSplitGroups * 128)) {
-        const int r = e / (BN / 4), c = (e % (BN / 4)) * 4;
-        if (m0 + r >= p.M || n0 + c >= p.N) continue;
-        float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-        for (int q = 0; q < splits; ++q) {
-            const float* part = cl.map_shared_rank(dyn, q) + r * BN + c;
-#pragma unroll
-            for (int g = 0; g < kSplitGroups; ++g) {
-                const float4 x = *reinterpret_cast<const float4*>(part + g * (BM * BN));
-                s.x += x.x; s.y += x.y; s.z += x.z; s.w += x.w;
+                for (int i = 0; i < 4; ++i) { acc[i][0] = fmaf(a[i], b.x, acc[i][0]); acc[i][1] = fmaf(a[i], b.y, acc[i][1]); }
             }
         }
-        float* dst = pp.c + (m0 + r) * p.c_sm + (n0 + c);
-        const float o[4] = {s.x * p.alpha, s.y * p.alpha, s.z * p.alpha, s.w * p.alpha};
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
 #pragma unroll
-        for (int j = 0; j < 4; ++j) if (n0 + c + j < p.N) dst[j] = o[j];
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+                if (arow + i < a_left && bcol + j < b_left) pp.c[(m0 + arow + i) * p.c_sm + n0 + bcol + j] = acc[i][j] * p.alpha;
     }
-    cl.sync();                                           // nobody leaves while a peer still reads
 }
 
 template <typename T, Fetch F, int WM, int WN, int TN, bool FUSED>
@@ -368,82 +393,25 @@ int launch_tile(const T* A, const T* B, float* C, const SimtContract& p, cudaStr
     return cudaGetLastError() == cudaSuccess ? ST_OK : ST_LAUNCH;
 }
 
-// CTAs per cluster: clusters beyond what the GPU's processor clusters hold at once wait for a second wave, so the size is the one
-// with the fewest slices one after the other (resident[S]: clusters of S that run together, 148 SMs: 74 of 2, 33 of 4, 15 of 8
-// and 7 of 16 with four groups, 33 of 8 and 14 of 16 with two).
-struct SplitPlan { int groups, splits; long long rounds; };
-inline void plan_split(SplitPlan& best, int groups, const int (&resident)[17], long long tiles, long long slices) {
-    for (int s = 1; s <= 16; ++s) {
-        if (resident[s] <= 0 || static_cast<long long>(s - 1) * groups >= slices) break;
-        const long long rounds = ((tiles + resident[s] - 1) / resident[s]) * ((slices + s * groups - 1) / (s * groups));
-        if (rounds < best.rounds) best = {groups, s, rounds};
-    }
+// at most half the SMs would have a 64 x 64 tile (so no extent of the launch below is large).  A CTA per SM takes 102 us for the 2601
+// tokens of a 64 x 64 tile; 64 such tiles (8 planes of 128 x 256) take 60 narrow, and 128 would take twice that.
+bool takes_narrow(const SimtContract& p) {
+    const bool plain = p.bias == nullptr && !p.clamp && p.opm_L == 0 && p.ln_stats == nullptr && p.gate == nullptr && p.act == 0;
+    return plain && p.a_sm == 1 && p.b_sn == 1 && p.c_sn == 1 && p.K >= 4 * kSlice && p.K <= 0x7fffffffLL &&
+           p.M <= 64LL * num_sms() && p.N <= 64LL * num_sms() && p.planes <= num_sms() &&
+           2 * ((p.M + 63) / 64) * ((p.N + 63) / 64) * p.planes <= num_sms();
 }
-
-template <typename T, Fetch F, int G>
-struct SplitKernel {
-    static constexpr int kThreads = G * 128, kSmem = G * 64 * 64 * static_cast<int>(sizeof(float));
-    static void config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute& at, dim3 grid, int splits, cudaStream_t st) {
-        cfg.gridDim = grid; cfg.blockDim = dim3(kThreads); cfg.dynamicSmemBytes = kSmem; cfg.stream = st;
-        at.id = cudaLaunchAttributeClusterDimension;
-        at.val.clusterDim.x = 1; at.val.clusterDim.y = 1; at.val.clusterDim.z = static_cast<unsigned>(splits);
-        cfg.attrs = &at; cfg.numAttrs = 1;
-    }
-    // clusters of each size that are resident together on the current device, asked once per device; null on an error
-    static const int (*resident(int dev))[17] {
-        static int table[64][17];
-        static std::once_flag once[64];
-        static bool ok[64];
-        std::call_once(once[dev], [&] {
-            auto kern = simt_contract_split_kernel<T, F, G>;
-            ok[dev] = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) == cudaSuccess &&
-                      cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
-            for (int s = 1; ok[dev] && s <= 16; ++s) {
-                cudaLaunchConfig_t cfg{};
-                cudaLaunchAttribute at{};
-                config(cfg, at, dim3(1, 1, static_cast<unsigned>(s)), s, nullptr);
-                int n = 0;
-                table[dev][s] = cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess ? n : 0;
-            }
-            cudaGetLastError();
-        });
-        return ok[dev] ? &table[dev] : nullptr;
-    }
-    static int launch(const T* A, const T* B, float* C, const SimtContract& p, int splits, cudaStream_t st) {
-        const int nt = static_cast<int>((p.N + 63) / 64);
-        cudaLaunchConfig_t cfg{};
-        cudaLaunchAttribute at{};
-        config(cfg, at, dim3(static_cast<unsigned>((p.M + 63) / 64 * nt), 1, static_cast<unsigned>(p.planes * splits)), splits, st);
-        if (cudaLaunchKernelEx(&cfg, simt_contract_split_kernel<T, F, G>, A, B, C, p, nt) != cudaSuccess) { cudaGetLastError(); return ST_LAUNCH; }
-        return ST_OK;
-    }
-};
-
-// ST_UNSUPPORTED_PATH: not worth a split
-template <typename T, Fetch F>
-int launch_split(const T* A, const T* B, float* C, const SimtContract& p, long long tiles, cudaStream_t st) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) { cudaGetLastError(); return ST_UNSUPPORTED_PATH; }
-    const auto* r2 = SplitKernel<T, F, 2>::resident(dev);
-    const auto* r4 = SplitKernel<T, F, 4>::resident(dev);
-    if (!r2 || !r4) return ST_UNSUPPORTED_PATH;
-    const long long slices = (p.K + kSlice - 1) / kSlice;
-    SplitPlan plan{1, 1, slices};
-    plan_split(plan, 2, *r2, tiles, slices);
-    plan_split(plan, 4, *r4, tiles, slices);
-    if (plan.groups == 1) return ST_UNSUPPORTED_PATH;
-    return plan.groups == 2 ? SplitKernel<T, F, 2>::launch(A, B, C, p, plan.splits, st) : SplitKernel<T, F, 4>::launch(A, B, C, p, plan.splits, st);
+template <int VEC>
+int launch_narrow(const float* A, const float* B, float* C, const SimtContract& p, cudaStream_t st) {
+    const int mt = static_cast<int>((p.M + kNarrowM - 1) / kNarrowM), nt = static_cast<int>((p.N + kNarrowN - 1) / kNarrowN);
+    simt_contract_narrow_kernel<VEC><<<dim3(static_cast<unsigned>(mt * nt), 1, static_cast<unsigned>(p.planes)), kNarrowThreads, 0, st>>>(A, B, C, p, nt);
+    return cudaGetLastError() == cudaSuccess ? ST_OK : ST_LAUNCH;
 }
 
 template <typename T, Fetch F>
 int launch_fetch(const T* A, const T* B, float* C, const SimtContract& p, cudaStream_t st) {
     const bool fused = p.ln_stats != nullptr || p.gate != nullptr || p.act != 0;
     const int sms = num_sms();
-    const long long small = ((p.M + 63) / 64) * ((p.N + 63) / 64) * p.planes;
-    if (p.may_split && !fused && 2 * small <= sms && p.K >= 4 * kSlice) {      // at most half the SMs would have a tile
-        const int rc = launch_split<T, F>(A, B, C, p, small, st);
-        if (rc != ST_UNSUPPORTED_PATH) return rc;
-    }
     if (p.N <= 32)
         return fused ? launch_tile<T, F, 4, 1, 4, true>(A, B, C, p, st) : launch_tile<T, F, 4, 1, 4, false>(A, B, C, p, st);
     // 64 x 128 tiles where there are enough of them to fill the SMs three deep, 64 x 64 below
@@ -462,6 +430,12 @@ int launch_typed(const T* A, const T* B, float* C, const SimtContract& p, cudaSt
     const bool base_ok = reinterpret_cast<uintptr_t>(A) % gb == 0 && reinterpret_cast<uintptr_t>(B) % gb == 0 &&
                          (p.ne2 == 1 || (p.a_s2 % 4 == 0 && p.b_s2 % 4 == 0)) &&
                          (p.planes == p.ne2 || (p.a_s3 % 4 == 0 && p.b_s3 % 4 == 0));
+    if constexpr (std::is_same_v<T, float>) {
+        if (takes_narrow(p)) {
+            const bool vec = base_ok && p.M % 4 == 0 && p.N % 4 == 0 && p.a_sk % 4 == 0 && p.b_sk % 4 == 0;
+            return vec ? launch_narrow<4>(A, B, C, p, st) : launch_narrow<1>(A, B, C, p, st);
+        }
+    }
     if (base_ok && p.a_sk == 1 && p.b_sk == 1 && p.K % 4 == 0 && p.a_sm % 4 == 0 && p.b_sn % 4 == 0)
         return launch_fetch<T, Fetch::VEC_K>(A, B, C, p, st);
     if (base_ok && p.a_sm == 1 && p.b_sn == 1 && p.M % 4 == 0 && p.N % 4 == 0 && p.a_sk % 4 == 0 && p.b_sk % 4 == 0)
@@ -489,7 +463,6 @@ int launch_simt_contract(const void* A, const void* B, float* C, const SimtContr
     }
     const bool c_al = (reinterpret_cast<uintptr_t>(C) & 15u) == 0 && p.N % 4 == 0 && (p.ne2 == 1 || p.c_s2 % 4 == 0) && (p.planes == p.ne2 || p.c_s3 % 4 == 0);
     p.vec_c = p.opm_L > 0 ? (c_al && p.opm_B == 1 && p.opm_L % 4 == 0) : (c_al && p.c_sn == 1 && p.c_sm % 4 == 0);
-    p.may_split = p.may_split && p.c_sn == 1 && p.bias == nullptr && !p.clamp && p.opm_L == 0;
     if (elem == 0) return launch_typed<float>(static_cast<const float*>(A), static_cast<const float*>(B), C, p, st);
     if (elem == 1) return launch_typed<__half>(static_cast<const __half*>(A), static_cast<const __half*>(B), C, p, st);
     return launch_typed<__nv_bfloat16>(static_cast<const __nv_bfloat16*>(A), static_cast<const __nv_bfloat16*>(B), C, p, st);

@@ -878,14 +878,28 @@ def test_exact_contraction_tile_edges(oracle, M, K, N):
 
 
 @pytest.mark.parametrize("n0,n1,K,p2,ne02", [(256, 128, 2601, 1, 1), (33, 32, 4099, 1, 1), (36, 132, 65, 2, 1), (8, 4, 64, 1, 1),
-                                             (130, 66, 1000, 3, 3), (64, 64, 16 * 64 + 1, 1, 1)])
-def test_exact_contraction_split(oracle, n0, n1, K, p2, ne02):
-    """Few output tiles and a long contraction: split over the groups of a CTA and the CTAs of a cluster.  Repeats give the
-    same bits (the parts are added in a fixed order)."""
+                                             (130, 66, 1000, 3, 3), (64, 64, 16 * 64 + 1, 1, 1), (512, 160, 100, 1, 1), (31, 17, 256, 40, 1)])
+def test_exact_contraction_small_result(oracle, n0, n1, K, p2, ne02):
+    """Few output tiles and a long contraction (narrow tiles): one ascending chain per output, bit for bit -- the same as the product of
+    the transposed operands through mul_mat and as each plane by itself -- with rows that are and are not whole groups of four."""
     s0, s1 = cases.out_prod_case(n0, n1, K, p2, 1, ne02=ne02, seed=32)
-    got = host(ops.out_prod_cuda(dev(s0), dev(s1), path=PATH_SIMT))
-    assert cases.rel_err(got, oracle.out_prod(s0, s1)) <= TOL_FP32
-    assert np.array_equal(got, host(ops.out_prod_cuda(dev(s0), dev(s1), path=PATH_SIMT)))
+    got = ops.out_prod_cuda(dev(s0), dev(s1), path=PATH_SIMT)
+    assert cases.rel_err(host(got), oracle.out_prod(s0, s1)) <= TOL_FP32
+    for i in {0, p2 - 1}:
+        t0, t1 = dev(s0[:, i * ne02 // p2]), dev(s1[:, i])                 # [1, K, n0], [1, K, n1]
+        assert torch.equal(got[0, i], ops.mul_mat_cuda(t1[0].t().contiguous(), t0[0].t().contiguous(), path=PATH_SIMT))
+        assert torch.equal(got[0, i], ops.out_prod_cuda(t0[None], t1[None], path=PATH_SIMT)[0, 0])
+
+
+def test_exact_contraction_is_one_ascending_chain():
+    """out_prod and mul_mat on the CUDA cores against the chain itself: acc = round(acc + a b), k ascending (the 64-bit mantissa holds
+    the product exactly and the sum to 40 bits beyond the rounding)."""
+    s0, s1 = cases.out_prod_case(36, 20, 700, 1, 1, seed=34)
+    acc = np.zeros((20, 36), np.float32)
+    for k in range(700):
+        acc = (acc.astype(np.longdouble) + s1[0, 0, k].astype(np.longdouble)[:, None] * s0[0, 0, k].astype(np.longdouble)[None]).astype(np.float32)
+    assert np.array_equal(host(ops.out_prod_cuda(dev(s0), dev(s1), path=PATH_SIMT))[0, 0], acc)
+    assert np.array_equal(host(ops.mul_mat_cuda(dev(s1[0, 0].T), dev(s0[0, 0].T), path=PATH_SIMT)), acc)
 
 
 @pytest.mark.parametrize("n0,n1,K,p2", [(256, 128, 2601, 1), (64, 256, 4096, 1), (36, 20, 300, 1), (100, 36, 1000, 1), (64, 160, 225, 2),
