@@ -1,7 +1,7 @@
 // umma_gemm.cu -- host side of the tcgen05 contraction engine: eligibility checks, tensor maps,
 // tile shape selection and the launch.
+#include <climits>
 #include <cstdlib>
-#include <mutex>
 #include "kernels.h"
 #include "tma_host.h"
 #include "umma_gemm.cuh"
@@ -79,73 +79,99 @@ int launch_bn_mn(int BN, bool half, const CUtensorMap& tmA, const CUtensorMap& t
     }
 }
 
-template <int BN>
-struct SplitGemm {
-    static void config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute& at, unsigned tiles, int splits, cudaStream_t st) {
-        cfg.gridDim = dim3(tiles, static_cast<unsigned>(splits)); cfg.blockDim = dim3(192); cfg.dynamicSmemBytes = gemm_split_smem_bytes<BN>();
-        cfg.stream = st;
-        at.id = cudaLaunchAttributeClusterDimension;
-        at.val.clusterDim.x = 1; at.val.clusterDim.y = static_cast<unsigned>(splits); at.val.clusterDim.z = 1;
-        cfg.attrs = &at; cfg.numAttrs = 1;
-    }
-    // clusters of each size that run together on the current device, asked once per device; null on an error
-    static const int (*resident(int dev))[17] {
-        static int table[64][17];
-        static std::once_flag once[64];
-        static bool ok[64];
-        std::call_once(once[dev], [&] {
-            auto kern = umma_gemm_split_kernel<BN>;
-            ok[dev] = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, gemm_split_smem_bytes<BN>()) == cudaSuccess &&
-                      cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
-            for (int s = 2; ok[dev] && s <= 16; ++s) {
-                cudaLaunchConfig_t cfg{};
-                cudaLaunchAttribute at{};
-                config(cfg, at, 1, s, nullptr);
-                int n = 0;
-                table[dev][s] = cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess ? n : 0;
-            }
-            cudaGetLastError();
-        });
-        return ok[dev] ? &table[dev] : nullptr;
-    }
-    static int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, GemmParams p, int box_a, int splits, cudaStream_t st) {
-        p.n_tiles = (p.N + BN - 1) / BN;
-        p.m_tiles = (p.M + 127) / 128;
-        cudaLaunchConfig_t cfg{};
-        cudaLaunchAttribute at{};
-        config(cfg, at, static_cast<unsigned>(p.m_tiles * p.n_tiles * p.batch), splits, st);
-        if (cudaLaunchKernelEx(&cfg, umma_gemm_split_kernel<BN>, tmA, tmB, p, box_a) != cudaSuccess) { cudaGetLastError(); return ST_LAUNCH; }
-        return ST_OK;
-    }
-};
+// ---- the contraction in parts (umma_gemm_split_kernel, umma_gemm_parts_kernel) -------------------------------------------
+// Clusters of S CTAs of the split kernel that a B200 holds at once (one CTA per SM, 148 SMs; cudaOccupancyMaxActiveClusters), index S.
+// Constants, so that the number of parts and with it the bits of a result follow from the extents alone.
+constexpr int kSplitSms = 148;
+constexpr int kSplitResident[17] = {0, 148, 74, 45, 33, 26, 22, 15, 15, 15, 11, 7, 7, 7, 7, 7, 7};
+constexpr long long kStepNs = 340;             // one K step of a CTA
 
-// Tile width and cluster size of the split form: the fewest operand bytes one after the other into an SM -- K steps of a CTA times
-// its rows, times the waves of clusters (what does not run together waits).  bn = 0: more than half the SMs have a tile of the
-// general kernel, or there are fewer than four K steps (256 x 256 over 256 tokens, eight of them: 11.7 -> 5.4 us; over 128: 9.4 -> 4.7).
-struct GemmSplit { int bn = 0, splits = 1; };
-template <int BN>
-void plan_gemm_split(GemmSplit& best, long long& cost, int dev, const UmmaGemmArgs& a, int k_steps) {
-    const int (*res)[17] = SplitGemm<BN>::resident(dev);
-    if (!res || (BN > 32 && a.N <= BN / 2)) return;
-    const long long tiles = static_cast<long long>((a.M + 127) / 128) * ((a.N + BN - 1) / BN) * a.batch;
-    const long long rows = (a.M < 128 ? a.M : 128) + (a.N < BN ? a.N : BN);
-    for (int s = 2; s <= 16 && s <= k_steps; ++s) {
-        if ((*res)[s] <= 0) continue;
-        const long long c = ((tiles + (*res)[s] - 1) / (*res)[s]) * ((k_steps + s - 1) / s) * rows;
-        if (c < cost) { cost = c; best.bn = BN; best.splits = s; }
-    }
-}
-GemmSplit gemm_split(const UmmaGemmArgs& a, int general_bn, int k_steps) {
-    GemmSplit g;
+template <typename Kernel>
+bool configure_once(Kernel kern, int smem, bool clusters, bool (&done)[64]) {
     int dev = 0;
-    if (!a.may_split || k_steps < 4 || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return g;
-    const long long tiles = static_cast<long long>((a.M + 127) / 128) * ((a.N + general_bn - 1) / general_bn) * a.batch;
-    if (2 * tiles > num_sms()) return g;
-    long long cost = static_cast<long long>(k_steps) * (128 + general_bn);
-    plan_gemm_split<128>(g, cost, dev, a, k_steps);
-    plan_gemm_split<64>(g, cost, dev, a, k_steps);
-    plan_gemm_split<32>(g, cost, dev, a, k_steps);
-    return g;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) { cudaGetLastError(); return false; }
+    if (done[dev]) return true;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
+        (clusters && cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)) {
+        cudaGetLastError();
+        return false;
+    }
+    return done[dev] = true;
+}
+
+template <int BN>
+int launch_split(const CUtensorMap& tmA, const CUtensorMap& tmB, GemmParams p, int box_a, int box_b, int parts, cudaStream_t st) {
+    static bool done[64] = {false};
+    auto kern = umma_gemm_split_kernel<BN>;
+    if (!configure_once(kern, gemm_split_smem_bytes<BN>(), true, done)) return ST_LAUNCH;
+    p.n_tiles = (p.N + BN - 1) / BN;
+    p.m_tiles = (p.M + 127) / 128;
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute at{};
+    cfg.gridDim = dim3(static_cast<unsigned>(p.m_tiles * p.n_tiles * p.batch), static_cast<unsigned>(parts));
+    cfg.blockDim = dim3(192); cfg.dynamicSmemBytes = gemm_split_smem_bytes<BN>(); cfg.stream = st;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = 1; at.val.clusterDim.y = static_cast<unsigned>(parts); at.val.clusterDim.z = 1;
+    cfg.attrs = &at; cfg.numAttrs = 1;
+    if (cudaLaunchKernelEx(&cfg, kern, tmA, tmB, p, box_a, box_b) != cudaSuccess) { cudaGetLastError(); return ST_LAUNCH; }
+    return ST_OK;
+}
+
+template <int BN>
+int launch_parts(const CUtensorMap& tmA, const CUtensorMap& tmB, GemmParams p, int box_a, int box_b, int parts, cudaStream_t st) {
+    static bool done[64] = {false};
+    auto kern = umma_gemm_parts_kernel<BN>;
+    if (!configure_once(kern, gemm_parts_smem_bytes<BN>(), false, done)) return ST_LAUNCH;
+    p.n_tiles = (p.N + BN - 1) / BN;
+    p.m_tiles = (p.M + 127) / 128;
+    const long long total = static_cast<long long>(p.m_tiles) * p.n_tiles * p.batch;
+    if (total > 0x7fffffffLL - num_sms()) return ST_BAD_ARGS;
+    const int grid = static_cast<int>(total < num_sms() ? total : num_sms());
+    kern<<<grid, 64 + 32 * kPartsEpiWarps<BN>, gemm_parts_smem_bytes<BN>(), st>>>(tmA, tmB, p, parts, box_a, box_b);
+    return cudaGetLastError() == cudaSuccess ? ST_OK : ST_LAUNCH;
+}
+
+// Time (ns) of `batch` results on clusters of S CTAs and tiles of BN columns: waves of clusters (what does not run together waits), each
+// with its launch, the sum over the cluster and the K steps of a CTA.  Fitted to 32 x 32 .. 512 x 256 over 128 .. 16384 tokens at
+// 1 .. 512 planes; the choice below was the faster form, or within 5 % of it, at all of them.
+long long split_ns(const UmmaGemmArgs& a, int batch, int BN, int S, int k_steps) {
+    if (BN > 32 && a.N <= BN / 2) return LLONG_MAX;
+    const long long tiles = static_cast<long long>((a.M + 127) / 128) * ((a.N + BN - 1) / BN) * batch;
+    return ((tiles + kSplitResident[S] - 1) / kSplitResident[S]) * (2900 + 27 * BN + kStepNs * ((k_steps + S - 1) / S));
+}
+// The same with all parts of a tile in one CTA: a part takes its K steps, or the time to add it to the sum where that is longer.
+long long parts_ns(const UmmaGemmArgs& a, int BN, int parts, int k_steps) {
+    const long long tiles = static_cast<long long>((a.M + 127) / 128) * ((a.N + BN - 1) / BN) * a.batch;
+    const long long steps = kStepNs * ((k_steps + parts - 1) / parts), add = 390 + 4 * BN / 5;
+    return 3600 + 14 * BN + ((tiles + kSplitSms - 1) / kSplitSms) * parts * (steps > add ? steps : add);
+}
+
+// Parts of the contraction, from M, N and K alone: the cluster size that is fastest for one result, at least two K steps per part (with
+// one, a CTA that computes all parts waits for its sums: 512 planes of 256 x 256 over 408 tokens 107 us in 13 parts, 88 undivided).
+// 1: more than half the SMs have a tile of the general kernel, or there are fewer than four K steps (256 x 256 over 256 tokens,
+// eight of them: 11.7 -> 5.4 us; over 128: 9.4 -> 4.7).
+int gemm_parts(const UmmaGemmArgs& a, int general_bn, int k_steps) {
+    const long long tiles = static_cast<long long>((a.M + 127) / 128) * ((a.N + general_bn - 1) / general_bn);
+    if (!a.may_split || k_steps < 4 || 2 * tiles > kSplitSms) return 1;
+    long long best = LLONG_MAX;
+    int parts = 1;
+    for (int s = 2; s <= 16 && 2 * s <= k_steps; ++s)
+        for (int BN : {32, 64, 128}) {
+            const long long ns = split_ns(a, 1, BN, s, k_steps);
+            if (ns < best) { best = ns; parts = s; }
+        }
+    return parts;
+}
+
+// Tile width of the split kernel for a whole call, or 0: all parts of a tile in one CTA.
+int split_width(const UmmaGemmArgs& a, int general_bn, int k_steps, int parts) {
+    long long best = parts_ns(a, general_bn, parts, k_steps);
+    int width = 0;
+    for (int BN : {32, 64, 128}) {
+        const long long ns = split_ns(a, a.batch, BN, parts, k_steps);
+        if (ns < best) { best = ns; width = BN; }
+    }
+    return width;
 }
 
 int pick_bn(int N) {
@@ -173,16 +199,11 @@ int launch_umma_gemm(const UmmaGemmArgs& a, cudaStream_t st) {
         // A[b][k][m], B[b][k][n] with the row index contiguous: fp32 operands become tf32 in the TMA unit and use
         // the 32-byte-chunk swizzle, 16-bit operands the ordinary 128-byte swizzle
         if (a.opm_L > 0) return ST_UNSUPPORTED_PATH;
-        CUtensorMap tmA, tmB;
         const bool half = a.elem != 0;
         const TmaType tt = !half ? TmaType::TF32 : (a.elem == 1 ? TmaType::F16 : TmaType::BF16);
         const uint32_t box = half ? 64 : 32;
         const uint64_t a_bs = (a.batch > 1) ? static_cast<uint64_t>(a.a_batch) * es : 0;
         const uint64_t b_bs = (a.batch > 1) ? static_cast<uint64_t>(a.b_batch) * es : 0;
-        if (!make_tmap_3d(&tmA, tt, a.A, a.M, a.K, a.batch, static_cast<uint64_t>(a.lda) * es, a_bs, box, box, half ? 1 : 2))
-            return ST_UNSUPPORTED_PATH;
-        if (!make_tmap_3d(&tmB, tt, a.B, a.N, a.K, a.batch, static_cast<uint64_t>(a.ldb) * es, b_bs, box, box, half ? 1 : 2))
-            return ST_UNSUPPORTED_PATH;
         GemmParams p{};
         p.M = a.M; p.N = a.N; p.K = a.K; p.batch = a.batch;
         p.k_steps = (a.K + bk - 1) / bk;
@@ -191,23 +212,31 @@ int launch_umma_gemm(const UmmaGemmArgs& a, cudaStream_t st) {
         p.bias = a.bias; p.alpha = a.alpha; p.clamp = a.clamp;
         p.err = err;
         p.vec_ok = ((reinterpret_cast<uintptr_t>(a.C) & 15u) == 0) && (a.ldc % 4 == 0) && (a.c_batch % 4 == 0) && (a.N % 4 == 0);
-        const GemmSplit g = half ? GemmSplit() : gemm_split(a, BN, p.k_steps);
-        if (g.bn != 0) {
-            int box_a = 0;
-            // whole row blocks: an operand as [batch][row block][k][32], whose box holds all row blocks of a stage (one
-            // issuing thread needs 60 to 80 ns per load: 256 x 256 over 65536 tokens 62 us with a box per row block)
-            if (a.M % 32 == 0 && a.N % 32 == 0) {
-                const uint32_t ba = a.M < 128 ? a.M / 32 : 4, bb = (a.N < g.bn ? a.N : g.bn) / 32;
-                CUtensorMap wa, wb;
-                if (make_tmap_4d(&wa, tt, a.A, 32, a.K, a.M / 32, a.batch, static_cast<uint64_t>(a.lda) * es, 128, a_bs, 32, 32, 2, ba) &&
-                    make_tmap_4d(&wb, tt, a.B, 32, a.K, a.N / 32, a.batch, static_cast<uint64_t>(a.ldb) * es, 128, b_bs, 32, 32, 2, bb)) {
-                    tmA = wa; tmB = wb;
-                    box_a = static_cast<int>(ba);
-                }
+        const int parts = half ? 1 : gemm_parts(a, BN, p.k_steps);
+        const int width = parts > 1 ? split_width(a, BN, p.k_steps, parts) : 0, bn = width ? width : BN;
+        CUtensorMap tmA, tmB;
+        // whole row blocks: an operand as [batch][row block][k][32], whose box holds all row blocks of a stage (one issuing thread
+        // needs 60 to 80 ns per load: 256 x 256 over 65536 tokens 62 us with a box per row block)
+        const int box_a = parts > 1 && a.M % 32 == 0 ? (a.M < 128 ? a.M / 32 : 4) : 0;
+        const int box_b = parts > 1 && a.N % 32 == 0 ? (a.N < bn ? a.N : bn) / 32 : 0;
+        auto map = [&](CUtensorMap* m, const void* base, int rows, long long pitch, uint64_t bs, int blocks) {
+            const uint64_t pb = static_cast<uint64_t>(pitch) * es;
+            return blocks ? make_tmap_4d(m, tt, base, 32, a.K, rows / 32, a.batch, pb, 128, bs, 32, 32, 2, blocks)
+                          : make_tmap_3d(m, tt, base, rows, a.K, a.batch, pb, bs, box, box, half ? 1 : 2);
+        };
+        if (!map(&tmA, a.A, a.M, a.lda, a_bs, box_a) || !map(&tmB, a.B, a.N, a.ldb, b_bs, box_b)) return ST_UNSUPPORTED_PATH;
+        if (parts > 1) {
+            switch (width) {
+                case 128: return launch_split<128>(tmA, tmB, p, box_a, box_b, parts, st);
+                case 64: return launch_split<64>(tmA, tmB, p, box_a, box_b, parts, st);
+                case 32: return launch_split<32>(tmA, tmB, p, box_a, box_b, parts, st);
             }
-            if (g.bn == 128) return SplitGemm<128>::launch(tmA, tmB, p, box_a, g.splits, st);
-            if (g.bn == 64) return SplitGemm<64>::launch(tmA, tmB, p, box_a, g.splits, st);
-            return SplitGemm<32>::launch(tmA, tmB, p, box_a, g.splits, st);
+            switch (BN) {
+                case 32: return launch_parts<32>(tmA, tmB, p, box_a, box_b, parts, st);
+                case 64: return launch_parts<64>(tmA, tmB, p, box_a, box_b, parts, st);
+                case 128: return launch_parts<128>(tmA, tmB, p, box_a, box_b, parts, st);
+                default: return launch_parts<256>(tmA, tmB, p, box_a, box_b, parts, st);
+            }
         }
         return launch_bn_mn(BN, half, tmA, tmB, p, st);
     }

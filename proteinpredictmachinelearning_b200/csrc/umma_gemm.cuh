@@ -438,14 +438,16 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 }
 
 // =============================================================================================
-// The split form for a long contraction with a small result (weight gradients: dW = dY^T X over the tokens), fp32 operands with
-// the row index contiguous.  A cluster of up to 16 CTAs shares one 128 x BN tile: CTA r takes the K steps r, r + S, ...
-// (neighbouring in memory at any time), leaves its accumulator in its shared memory, and the CTAs add the parts piece by piece
-// in rank order over distributed shared memory -- no workspace, no atomics.  Partial sums stay fp32.
+// A long contraction with a small result (weight gradients: dW = dY^T X over the tokens), fp32 operands with the row index
+// contiguous.  The contraction is computed in S parts: part r is one accumulator over the K steps r, r + S, ... (neighbouring in memory
+// at any time), and the result is ((part 0 + part 1) + ...) in fp32 -- no workspace, no atomics.  S follows from M, N and K alone, so
+// the bits do not depend on how many batches a call holds; where the parts run does:
+//   umma_gemm_split_kernel  a cluster of S CTAs shares one 128 x BN tile, a part each, and adds them over distributed shared memory;
+//   umma_gemm_parts_kernel  with enough tiles for the SMs, a CTA computes all parts of a tile one after the other.
 //
-// Bound: operand bytes into each SM -- a CTA reads (128 + BN) * 4 bytes per token it owns, at most 16 CTAs share a tile
-// (64 SMs for 256 x 256: 93 GB/s each).  One CTA per tile, as the general kernel runs it, left 146 SMs idle: 256 x 256 over
-// 65536 tokens 1181 -> 45 us (134 MB: 21 us at copy bandwidth), 64 x 32 747 -> 41, 256 x 128 over 2601 41 -> 7.5.
+// Bound of the split form: operand bytes into each SM -- a CTA reads (128 + BN) * 4 bytes per token it owns, at most 16 CTAs share a
+// tile (64 SMs for 256 x 256: 93 GB/s each).  One CTA per tile left 146 SMs idle: 256 x 256 over 65536 tokens 1181 -> 45 us (134 MB:
+// 21 us at copy bandwidth), 64 x 32 747 -> 41, 256 x 128 over 2601 41 -> 7.5.
 // =============================================================================================
 template <int BN>
 __host__ __device__ constexpr int gemm_split_smem_bytes() { return gemm_num_stages<BN>() * gemm_stage_bytes<BN>() + 1024 + 512; }
@@ -453,7 +455,7 @@ __host__ __device__ constexpr int gemm_split_smem_bytes() { return gemm_num_stag
 template <int BN>
 __global__ void __launch_bounds__(192, 1)
 umma_gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmParams p,
-                       int box_a /* row blocks of 32 in a 4-D box of A (both maps are 4-D then); 0: 3-D maps, a box per row block */) {
+                       int box_a, int box_b /* row blocks of 32 in a 4-D box of the operand; 0: a 3-D map, a box per row block */) {
     constexpr int STAGES = gemm_num_stages<BN>();
     constexpr int STAGE_BYTES = gemm_stage_bytes<BN>();
     constexpr int BK = 32, kBox = BK * 128;
@@ -502,20 +504,18 @@ umma_gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
             // only boxes that hold rows of the operand: what the others' part of the stage contains reaches only accumulator rows
             // and columns outside the result
             const int na = box_a ? box_a : min(128 / BK, (p.M - row0 + BK - 1) / BK);
-            const int nb = box_a ? min(BN, p.N) / BK : min(BN / BK, (p.N - col0 + BK - 1) / BK);
+            const int nb = box_b ? box_b : min(BN / BK, (p.N - col0 + BK - 1) / BK);
             uint32_t it = 0;
             for (int ks = rank; ks < p.k_steps; ks += splits, ++it) {
                 const int s = it % STAGES;
                 if (!mbar_wait(empty_bar(s), ((it / STAGES) & 1u) ^ 1u, cta_abort, p.err, 0x111)) break;
                 const uint32_t sa = smem_base + s * STAGE_BYTES;
                 mbar_arrive_expect_tx(full_bar(s), static_cast<uint32_t>(na + nb) * kBox);
-                if (box_a) {                             // all row blocks of an operand with one instruction
-                    tma_load_4d(sa, &tmA, full_bar(s), 0, ks * BK, row0 / BK, b);
-                    tma_load_4d(sa + kGemmStageA, &tmB, full_bar(s), 0, ks * BK, col0 / BK, b);
-                    continue;
-                }
-                for (int i = 0; i < na; ++i) tma_load_3d(sa + i * kBox, &tmA, full_bar(s), row0 + i * BK, ks * BK, b);
-                for (int i = 0; i < nb; ++i) tma_load_3d(sa + kGemmStageA + i * kBox, &tmB, full_bar(s), col0 + i * BK, ks * BK, b);
+                // all row blocks of an operand with one instruction, where it has whole ones
+                if (box_a) tma_load_4d(sa, &tmA, full_bar(s), 0, ks * BK, row0 / BK, b);
+                else for (int i = 0; i < na; ++i) tma_load_3d(sa + i * kBox, &tmA, full_bar(s), row0 + i * BK, ks * BK, b);
+                if (box_b) tma_load_4d(sa + kGemmStageA, &tmB, full_bar(s), 0, ks * BK, col0 / BK, b);
+                else for (int i = 0; i < nb; ++i) tma_load_3d(sa + kGemmStageA + i * kBox, &tmB, full_bar(s), col0 + i * BK, ks * BK, b);
             }
         }
         __syncwarp();
@@ -578,6 +578,176 @@ umma_gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
         }
     }
     cl.sync();                                            // nobody leaves while a peer still reads
+    if (warp == 1) {
+        tc_fence_after();
+        tmem_dealloc(tmem_base, TMEM_COLS);
+    }
+}
+
+// All parts of a tile in one CTA, which walks the tiles as umma_gemm_kernel does.  The two accumulators in TMEM alternate between the
+// parts, so the epilogue warps (two per lane quarter from BN = 64 on, half of the columns each) add one to the sum in their registers while
+// the next is computed; the sum leaves through a transposition buffer.
+constexpr int kPartsPitch = 80;                           // bytes per staged row: 16 floats + 16 bytes of padding
+template <int BN> constexpr int kPartsEpiWarps = BN >= 64 ? 8 : 4;
+template <int BN>
+__host__ __device__ constexpr int gemm_parts_smem_bytes() {
+    return gemm_num_stages<BN>() * gemm_stage_bytes<BN>() + 1024 + 512 + kPartsEpiWarps<BN> * 32 * kPartsPitch;
+}
+
+template <int BN>
+__global__ void __launch_bounds__(64 + 32 * kPartsEpiWarps<BN>, 1)
+umma_gemm_parts_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmParams p, int parts, int box_a,
+                       int box_b) {
+    constexpr int STAGES = gemm_num_stages<BN>();
+    constexpr int STAGE_BYTES = gemm_stage_bytes<BN>();
+    constexpr int BK = 32, kBox = BK * 128;
+    constexpr int kEpi = kPartsEpiWarps<BN>, kCols = BN * 4 / kEpi;        // columns per epilogue warp
+    constexpr uint32_t TMEM_COLS = 2 * BN;
+    static_assert(gemm_parts_smem_bytes<BN>() <= 227 * 1024, "shared memory of an SM");
+
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
+    const uint32_t bar_base = smem_base + STAGES * STAGE_BYTES;
+    auto full_bar = [&](int s) { return bar_base + 8u * s; };
+    auto empty_bar = [&](int s) { return bar_base + 8u * (kGemmMaxStages + s); };
+    auto tfull_bar = [&](int a) { return bar_base + 8u * (2 * kGemmMaxStages + a); };
+    auto tempty_bar = [&](int a) { return bar_base + 8u * (2 * kGemmMaxStages + 2 + a); };
+    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + STAGES * STAGE_BYTES + 8 * (2 * kGemmMaxStages + 4));
+    volatile int* cta_abort = reinterpret_cast<volatile int*>(smem_gen + STAGES * STAGE_BYTES + 8 * (2 * kGemmMaxStages + 4) + 8);
+
+    const int warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < STAGES; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
+        for (int a = 0; a < 2; ++a) { mbar_init(tfull_bar(a), 1); mbar_init(tempty_bar(a), kEpi); }
+        *cta_abort = 0;
+        fence_barrier_init();
+    }
+    if (warp == 1) {
+        tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), TMEM_COLS);
+        tmem_relinquish();
+    }
+    if (warp == 0 && lane == 0) { prefetch_tmap(&tmA); prefetch_tmap(&tmB); }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+    const int tiles_per_batch = p.m_tiles * p.n_tiles, total = tiles_per_batch * p.batch;
+
+    if (warp == 0) {
+        if (lane == 0) {
+            uint32_t it = 0;
+            bool ok = true;
+            for (int t = blockIdx.x; ok && t < total; t += gridDim.x) {
+                const int b = t / tiles_per_batch, r_ = t - b * tiles_per_batch, mt = r_ / p.n_tiles;
+                const int row0 = mt * 128, col0 = (r_ - mt * p.n_tiles) * BN;
+                const int na = box_a ? box_a : min(128 / BK, (p.M - row0 + BK - 1) / BK);      // as in the split form
+                const int nb = box_b ? box_b : min(BN / BK, (p.N - col0 + BK - 1) / BK);
+                for (int r = 0; ok && r < parts; ++r)
+                    for (int ks = r; ks < p.k_steps; ks += parts, ++it) {
+                        const int s = it % STAGES;
+                        if (!mbar_wait(empty_bar(s), ((it / STAGES) & 1u) ^ 1u, cta_abort, p.err, 0x121)) { ok = false; break; }
+                        const uint32_t sa = smem_base + s * STAGE_BYTES;
+                        mbar_arrive_expect_tx(full_bar(s), static_cast<uint32_t>(na + nb) * kBox);
+                        if (box_a) tma_load_4d(sa, &tmA, full_bar(s), 0, ks * BK, row0 / BK, b);
+                        else {
+#pragma unroll
+                            for (int i = 0; i < 128 / BK; ++i) if (i < na) tma_load_3d(sa + i * kBox, &tmA, full_bar(s), row0 + i * BK, ks * BK, b);
+                        }
+                        if (box_b) tma_load_4d(sa + kGemmStageA, &tmB, full_bar(s), 0, ks * BK, col0 / BK, b);
+                        else {
+#pragma unroll
+                            for (int i = 0; i < BN / BK; ++i) if (i < nb) tma_load_3d(sa + kGemmStageA + i * kBox, &tmB, full_bar(s), col0 + i * BK, ks * BK, b);
+                        }
+                    }
+            }
+        }
+        __syncwarp();
+    } else if (warp == 1) {
+        if (lane == 0) {
+            const uint32_t idesc = make_idesc(1, 2, 2, 1, 1, 128, BN);
+            uint32_t it = 0, part = 0;
+            bool ok = true;
+            for (int t = blockIdx.x; ok && t < total; t += gridDim.x)
+                for (int r = 0; ok && r < parts; ++r, ++part) {
+                    const int acc = part & 1;
+                    if (!mbar_wait(tempty_bar(acc), ((part >> 1) & 1u) ^ 1u, cta_abort, p.err, 0x221)) { ok = false; break; }
+                    tc_fence_after();
+                    for (int ks = r; ks < p.k_steps; ks += parts, ++it) {
+                        const int s = it % STAGES;
+                        if (!mbar_wait(full_bar(s), (it / STAGES) & 1u, cta_abort, p.err, 0x222)) { ok = false; break; }
+                        tc_fence_after();
+                        const uint32_t sa = smem_base + s * STAGE_BYTES;
+                        const uint64_t da = make_smem_desc(sa, BK * 128, 512, kLayoutSW128Base32);
+                        const uint64_t db = make_smem_desc(sa + kGemmStageA, BK * 128, 512, kLayoutSW128Base32);
+#pragma unroll
+                        for (int kk = 0; kk < 4; ++kk)
+                            umma<MmaKind::TF32>(tmem_base + acc * BN, da + 64u * kk, db + 64u * kk, idesc, (ks != r || kk != 0) ? 1u : 0u);
+                        umma_commit(empty_bar(s));
+                    }
+                    if (ok) umma_commit(tfull_bar(acc));
+                }
+        }
+        __syncwarp();
+    } else {
+        const int q = warp & 3, first = kEpi == 8 ? ((warp - 2) >> 2) * kCols : 0;       // TMEM lane quarter; first column of the tile
+        uint8_t* stage = smem_gen + STAGES * STAGE_BYTES + 512 + (warp - 2) * (32 * kPartsPitch);
+        uint32_t part = 0;
+        bool ok = true;
+        for (int t = blockIdx.x; ok && t < total; t += gridDim.x) {
+            const int b = t / tiles_per_batch, r_ = t - b * tiles_per_batch, mt = r_ / p.n_tiles;
+            const int row0 = mt * 128 + q * 32, col0 = (r_ - mt * p.n_tiles) * BN + first;
+            float sum[kCols];
+#pragma unroll
+            for (int j = 0; j < kCols; ++j) sum[j] = 0.0f;
+            for (int r = 0; r < parts; ++r, ++part) {
+                const int acc = part & 1;
+                if (!mbar_wait(tfull_bar(acc), (part >> 1) & 1u, cta_abort, p.err, 0x321)) { ok = false; break; }
+                tc_fence_after();
+#pragma unroll
+                for (int c = 0; c < kCols / 32; ++c) {
+                    uint32_t v[32];
+                    tmem_ld32(tmem_base + acc * BN + first + c * 32 + (static_cast<uint32_t>(q * 32) << 16), v);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) sum[c * 32 + j] += __uint_as_float(v[j]);
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(tempty_bar(acc));
+            }
+            if (!ok) break;
+            float* C = p.C + static_cast<long long>(b) * p.c_batch;
+#pragma unroll
+            for (int c = 0; c < kCols / 16; ++c) {
+                if (col0 + c * 16 >= p.N) break;          // the same for every lane
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    *reinterpret_cast<float4*>(stage + lane * kPartsPitch + j * 16) =
+                        make_float4(sum[c * 16 + 4 * j] * p.alpha, sum[c * 16 + 4 * j + 1] * p.alpha, sum[c * 16 + 4 * j + 2] * p.alpha, sum[c * 16 + 4 * j + 3] * p.alpha);
+                __syncwarp();
+                const int col = col0 + c * 16 + (lane & 3) * 4;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {             // four lanes per row, eight rows at a time
+                    const int rr = (lane >> 2) + 8 * i;
+                    const float4 x = *reinterpret_cast<const float4*>(stage + rr * kPartsPitch + (lane & 3) * 16);
+                    if (row0 + rr >= p.M || col >= p.N) continue;
+                    float* dst = C + static_cast<long long>(row0 + rr) * p.ldc + col;
+                    if (p.vec_ok) *reinterpret_cast<float4*>(dst) = x;
+                    else {
+                        dst[0] = x.x;
+                        if (col + 1 < p.N) dst[1] = x.y;
+                        if (col + 2 < p.N) dst[2] = x.z;
+                        if (col + 3 < p.N) dst[3] = x.w;
+                    }
+                }
+                __syncwarp();
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();                                      // every role, also after an aborted wait
     if (warp == 1) {
         tc_fence_after();
         tmem_dealloc(tmem_base, TMEM_COLS);

@@ -913,6 +913,21 @@ def test_out_prod_split_on_tensor_cores(oracle, n0, n1, K, p2):
     assert np.array_equal(got, host(ops.out_prod_cuda(dev(s0), dev(s1), path=PATH_UMMA)))
 
 
+@pytest.mark.parametrize("n0,n1,K,P", [(256, 256, 2601, 40), (64, 160, 225, 200), (32, 32, 128, 600), (128, 128, 408, 160), (260, 132, 700, 60), (256, 256, 128, 64),
+                                       (36, 100, 97, 300), (1000, 520, 300, 8)])
+def test_out_prod_bits_do_not_depend_on_the_planes(n0, n1, K, P):
+    """tf32 out_prod: a plane gives the same bits alone, among a few and among many (the parts of the contraction on a cluster or in one
+    CTA, tiles of any width), and both are within tf32 of the 64-bit product."""
+    g = torch.Generator(device="cuda").manual_seed(35)
+    s0, s1 = (torch.randn((1, P, K, n), device="cuda", generator=g) for n in (n0, n1))
+    whole = ops.out_prod_cuda(s0, s1, path=PATH_UMMA)
+    ref = s1[0].double().transpose(1, 2) @ s0[0].double()
+    assert float((whole[0] - ref).abs().max() / ref.abs().max()) <= TOL_TF32
+    for lo, n in ((0, 1), (P // 2, 1), (P - 1, 1), (0, 3), (1, P // 2)):
+        part = ops.out_prod_cuda(s0[:, lo:lo + n].contiguous(), s1[:, lo:lo + n].contiguous(), path=PATH_UMMA)
+        assert torch.equal(part, whole[:, lo:lo + n]), (lo, n)
+
+
 def test_attention_full_size_properties():
     """The full-size attention case (MSA depth 256, L = 256, 8 heads x 32, shared pair bias): the tensor-core kernel
     agrees with the CUDA-core kernel, a permutation of the batch permutes the output, and exp(LSE) equals the
