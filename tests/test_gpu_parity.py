@@ -190,6 +190,27 @@ def test_linear_with_layernorm_and_gate_fused(oracle, M, K, N, path, tol):
     assert cases.rel_err(got, np.maximum(plain, 0)) <= tol
 
 
+@pytest.mark.parametrize("M,K,N", [(28481, 32, 132), (28481, 36, 128), (28480, 20, 100), (255, 36, 32), (129, 64, 20), (300, 33, 65), (64, 32, 70)])
+def test_exact_linear_with_layernorm_and_gate_tile_edges(M, K, N):
+    """The fused epilogue of the exact contraction on all its tiles (64 x 128 from 444 tiles on, 64 x 64, 128 x 32), with vector and
+    element-wise gate reads and stores: every row against the 64-bit product.  The gate starts 4 bytes off a 16-byte boundary where
+    that is accepted (N no multiple of 4)."""
+    shift = 1 if N % 4 else 0
+    g = torch.Generator(device="cuda").manual_seed(36)
+    x, w, u, v = (torch.randn(s, device="cuda", generator=g) for s in ((M, K), (N, K), (N,), (N,)))
+    gate = torch.randn(M * N + shift, device="cuda", generator=g)[shift:].view(M, N)
+    stats = torch.stack([0.3 * torch.randn(M, device="cuda", generator=g), 0.5 + torch.rand(M, device="cuda", generator=g)], 1).contiguous()
+    lin = (x.double() @ w.double().t() - stats[:, :1].double() * u.double()) * stats[:, 1:].double() + v.double()
+    act = {"none": lambda t: t, "sigmoid": torch.sigmoid, "silu": torch.nn.functional.silu, "tanh": torch.tanh, "relu": torch.relu}
+    for kind, f in act.items():
+        got = ops.mul_mat_fused(x, w, bias=v, ln_stats=stats, ln_u=u, gate=gate, act=kind, path=PATH_SIMT).double()
+        ref = f(lin) * gate.double()
+        assert float((got - ref).abs().max() / ref.abs().max()) <= TOL_FP32, kind
+    got = ops.mul_mat_fused(x, w, bias=v, act="silu", path=PATH_SIMT).double()
+    ref = torch.nn.functional.silu(x.double() @ w.double().t() + v.double())
+    assert float((got - ref).abs().max() / ref.abs().max()) <= TOL_FP32
+
+
 def test_row_stats_follow_op_norm(oracle):
     r = np.random.default_rng(3)
     x = (r.standard_normal((1000, 256)) * 2 + 3).astype(np.float32)
