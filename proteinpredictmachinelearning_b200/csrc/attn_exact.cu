@@ -219,6 +219,17 @@ int launch_attn_exact(const void* Q, const void* K, const void* V, int elem, con
     const long long here = static_cast<long long>((L + 63) / 64 * 64LL) * ((Lk + 63) / 64 * 64LL);
     const long long there = static_cast<long long>((L + 15) / 16 * 16LL) * ((Lk + 31) / 32 * 32LL);
     if (here > 2 * there) return ST_UNSUPPORTED_PATH;
+    // at a ratio of 2 itself the head dims with an unrolled instance there (32, 64) still lose in two places:
+    // one tile of 32 keys, as long as that kernel runs in one wave of 6 CTAs per SM (64 (batch, head)s of 128 rows and 32 keys, head dim
+    // 32: 1.19 times its time here; 148 of them, two waves there, 0.67);
+    // head dim 64, with two CTAs per SM here, when the second wave is less than half full (32 rows, 408 (batch, head)s: 1.17 times with
+    // 64 keys, 1.09 with 256; 296 and 450 of them 0.66 to 0.78; 512 keys 0.76, K and V no longer staying in L2 there)
+    if ((d == 32 || d == 64) && here == 2 * there) {
+        const long long bh = static_cast<long long>(B) * H, sms = num_sms();
+        const long long ctas = (L + 63) / 64 * bh, ctas_there = (L + 15) / 16 * bh;
+        if (Lk <= 32 && ctas_there <= 6 * sms) return ST_UNSUPPORTED_PATH;
+        if (d == 64 && Lk <= 256 && ctas > 2 * sms && ctas < 3 * sms) return ST_UNSUPPORTED_PATH;
+    }
     ExactAttn p;
     p.H = H; p.L = L; p.Lk = Lk; p.d = d; p.causal = causal; p.ft = ft; p.scale = scale; p.eps = eps;
     p.bias_batch_stride = bias_batch_stride; p.lay = lay;

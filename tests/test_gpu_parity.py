@@ -667,6 +667,16 @@ def test_attention_backward_short(oracle, B, h, L, d, causal, bias):
         assert torch.equal(ops.flash_attn_backward_cuda(*args, db, scale=0.2, causal=causal, want=(n,))[n], got[n]), n
 
 
+@pytest.mark.parametrize("B,h,L,Lk,d", [(2, 2, 128, 32, 32), (4, 2, 64, 30, 64), (37, 8, 192, 32, 32), (38, 8, 32, 64, 64), (37, 8, 32, 64, 64), (56, 8, 20, 250, 64),
+                                        (41, 8, 17, 257, 64)])
+def test_attention_exact_half_empty_tiles(oracle, B, h, L, Lk, d):
+    """Twice the scores of the 16-row kernel's tiles: both sides of the rule between the two."""
+    Q, K, V, bi = cases.attn_case(B, h, L, d, Lk=Lk, seed=26, bias_bcast=True)
+    O, LSE = ops.flash_attn_forward_cuda(dev(Q), dev(K), dev(V), dev(bi), scale=0.2, bias_bcast=True, path=PATH_SIMT)
+    rO, rL = oracle.flash_attn(Q, K, V, bi, scale=0.2, bias_bcast=True)
+    assert cases.rel_err(host(O), rO) <= TOL_FP32 and np.abs(host(LSE) - rL).max() <= 1e-5
+
+
 @pytest.mark.parametrize("d,dtype", [(32, None), (64, None), (20, None), (32, torch.bfloat16)])
 def test_attention_exact_causal_ignores_what_a_row_does_not_see(d, dtype):
     """Infinities and NaNs in V of later keys of the same tile: the rows before them keep their bits."""
