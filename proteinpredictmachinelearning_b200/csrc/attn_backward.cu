@@ -81,7 +81,7 @@ __device__ __forceinline__ void store_rows(float* dst, const float* red, int r0,
     }
 }
 
-// four neighbours of a row of [L] floats from column c on, or `fill` past L
+// four neighbours of a row of [L] floats from column c on, zero past L
 __device__ __forceinline__ float4 row4(const float* row, int c, int L, bool vec) {
     if (vec) return c < L ? attn_ld4(row + c) : make_float4(0.f, 0.f, 0.f, 0.f);
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);

@@ -581,9 +581,9 @@ def test_attention_first_key_tile_masked(oracle, d, L, Lk, path):
     (2, 3, 45, 32, True, False, False, ()),          # causal, no bias (golden)
     (2, 8, 51, 32, False, True, True, ()),           # dev size, one bias for every batch
     (3, 8, 100, 8, False, True, False, (0,)),        # extra-MSA heads
-    (2, 2, 70, 64, True, True, False, ()),           # d = 64 (two channels per lane), causal with bias
+    (2, 2, 70, 64, True, True, False, ()),           # d = 64, causal with bias
     (1, 4, 256, 32, False, True, True, ()),          # main-track size of one batch
-    (2, 2, 33, 20, False, False, False, ()),         # a head dim that is no power of two, one row past a tile
+    (2, 2, 33, 20, False, False, False, ()),         # a head dim that is no power of two, one row more than the short form takes
 ])
 def test_attention_backward(oracle, B, h, L, d, causal, bias, bcast, masked):
     """flash_attn_backward against the restated CPU routine of the reference (src/ops/FlashAttn.cpp:144-216) on the
@@ -712,6 +712,24 @@ def test_attention_backward_causal_ignores_what_a_row_does_not_see(d):
         assert torch.equal(got["dQ"][:, :, :j], ref["dQ"][:, :, :j]) and torch.equal(got["dQ"][:, :, j + 1:], ref["dQ"][:, :, j + 1:]), j
 
 
+@pytest.mark.parametrize("which", ["in", "bias", "out", "dbias"])
+def test_attention_backward_bases_off_16_bytes(which):
+    """Rows in whole groups of four whose base lies 4 bytes off a 16-byte boundary: element-wise access by the address alone; the bits
+    do not change."""
+    Q, K, V, bi, dO = cases.attn_backward_case(1, 2, 68, 32, seed=27)
+    def shifted(x, off):
+        t = torch.zeros(x.numel() + 1, device="cuda")
+        t[off:off + x.numel()] = x.flatten()
+        return t[off:off + x.numel()].view(x.shape)
+    q, k, v, b, do = (dev(x) for x in (Q, K, V, bi, dO))
+    o, lse = ops.flash_attn_forward_cuda(q, k, v, b, scale=0.2, path=PATH_SIMT)
+    ref = ops.flash_attn_backward_cuda(q, k, v, o, do, lse, b, scale=0.2)
+    out = {n: shifted(torch.zeros_like(t), int(which == ("dbias" if n == "dbias" else "out"))) for n, t in ref.items()}
+    ops.flash_attn_backward_cuda(shifted(q, int(which == "in")), k, v, o, do, lse, shifted(b, int(which == "bias")), scale=0.2, out=out)
+    for n in ref:
+        assert torch.equal(out[n], ref[n]), n
+
+
 def test_attention_backward_from_the_cuda_forward(oracle):
     """Forward on the tensor cores, backward on its O and LSE: the chain a training step runs (1e-3: the forward is tf32)."""
     Q, K, V, bi, dO = cases.attn_backward_case(2, 8, 128, 32, seed=9, bias_bcast=True)
@@ -751,7 +769,11 @@ def test_backward_shapes_of_a_linear(oracle):
     (4, 8, 100, 8, None, True, PATH_SIMT, TOL_FP32, 1e-5),       # extra-MSA heads (d = 8): thread-per-row kernel
     (5, 8, 100, 8, None, True, PATH_AUTO, TOL_TF32, 2e-3),       # extra-MSA heads (d = 8): warp-level tensor-core kernel
     (5, 8, 1, 8, 64, False, PATH_AUTO, TOL_FP32, 1e-5),          # global column attention: one query, keys over lanes
-    (2, 4, 70, 64, 44, True, PATH_AUTO, TOL_FP32, 1e-5),         # generic kernel
+    (2, 4, 70, 64, 44, True, PATH_AUTO, TOL_FP32, 1e-5),         # exact kernel on 64 x 64 tiles
+    (2, 2, 100, 41, 90, True, PATH_AUTO, TOL_FP32, 1e-5),        # the same, rows that are no whole groups of four
+    (2, 4, 70, 64, None, True, PATH_SIMT, TOL_FP32, 1e-5),       # 16-row kernel: just past a tile, head dim unrolled
+    (2, 4, 70, 20, None, True, PATH_SIMT, TOL_FP32, 1e-5),       # the same, head dim at run time
+    (2, 2, 33, 96, 50, False, PATH_AUTO, TOL_FP32, 1e-5),        # 16-row kernel: a head dim above 64
 ])
 def test_attention_on_token_major_operands_with_gate(oracle, B, h, L, d, Lk, bias, path, tol, ltol):
     """The projections' outputs as they lie ([B][L][h*d], here as column ranges of one fused [B][L][4*h*d] buffer) in,
@@ -903,9 +925,30 @@ def test_exact_contraction_tile_edges(oracle, M, K, N):
     """Edges of the exact contraction's tiles (64 x 64, 64 x 128 from 444 tiles on, 128 x 32) and of its slices of 16, with
     vector and element-wise loads and stores."""
     a, b, bi = cases.mul_mat_case(M, K, N, seed=31)
-    got = host(ops.mul_mat_cuda(dev(a), dev(b), dev(bi), path=PATH_SIMT))
+    got = ops.mul_mat_cuda(dev(a), dev(b), dev(bi), path=PATH_SIMT)
     rows = np.unique(np.r_[0:min(M, 200), max(0, M - 200):M])
-    assert cases.rel_err(got[rows], oracle.mul_mat_f32(np.ascontiguousarray(a[rows]), b, bi)) <= TOL_FP32
+    assert cases.rel_err(host(got)[rows], oracle.mul_mat_f32(np.ascontiguousarray(a[rows]), b, bi)) <= TOL_FP32
+    ref = dev(a).double() @ dev(b).double().t() + dev(bi).double()             # every row
+    assert float((got - ref).abs().max() / ref.abs().max()) <= TOL_FP32
+
+
+@pytest.mark.parametrize("M,K,N", [(130, 64, 128), (28480, 20, 132), (256, 256, 128)])
+@pytest.mark.parametrize("sa,sb,sc", [(1, 0, 0), (0, 1, 0), (0, 0, 1)])
+def test_exact_contraction_bases_off_16_bytes(M, K, N, sa, sb, sc):
+    """Extents in whole groups of four with one base 4 bytes off: element-wise loads, or stores, by the address alone; the bits do not
+    change.  Last case: out_prod over 256 tokens (narrow tiles) as well."""
+    g = torch.Generator(device="cuda").manual_seed(37)
+    a, b, c = (torch.zeros(m * n + 1, device="cuda") for m, n in ((M, K), (N, K), (M, N)))
+    a[sa:sa + M * K] = torch.randn(M * K, device="cuda", generator=g)
+    b[sb:sb + N * K] = torch.randn(N * K, device="cuda", generator=g)
+    va, vb, vc = a[sa:sa + M * K].view(M, K), b[sb:sb + N * K].view(N, K), c[sc:sc + M * N].view(M, N)
+    ref = ops.mul_mat_cuda(va.clone(), vb.clone(), path=PATH_SIMT)
+    assert torch.equal(ops.mul_mat_cuda(va, vb, path=PATH_SIMT, out=vc), ref)
+    assert float((ref - va.double() @ vb.double().t()).abs().max() / ref.abs().max()) <= TOL_FP32
+    if M == K:
+        at = a[sa:sa + M * K].view(1, 1, K, M)                                  # read as [K][M], [K][N]
+        bt = b[sb:sb + N * K].view(1, 1, K, N)
+        assert torch.equal(ops.out_prod_cuda(at, bt, path=PATH_SIMT), ops.out_prod_cuda(at.clone(), bt.clone(), path=PATH_SIMT))
 
 
 @pytest.mark.parametrize("n0,n1,K,p2,ne02", [(256, 128, 2601, 1, 1), (33, 32, 4099, 1, 1), (36, 132, 65, 2, 1), (8, 4, 64, 1, 1),
