@@ -29,7 +29,8 @@ extern "C" {
 
 /* kernel family selectors ("path" arguments) */
 #define PPML_B200_PATH_AUTO 0   /* tensor cores when the shape allows, else CUDA cores */
-#define PPML_B200_PATH_SIMT 1   /* CUDA cores only (exact fp32 accumulation order)      */
+#define PPML_B200_PATH_SIMT 1   /* CUDA cores only, fp32 throughout; every product one chain of fused multiply-adds with k
+                                 * ascending, the reference's order, but for ppml_b200_out_prod (see there) */
 #define PPML_B200_PATH_UMMA 2   /* tcgen05 only; status 7 when the shape is not eligible */
 
 /* how fp32 operands become tf32 on the tensor-core path */
@@ -241,11 +242,21 @@ int ppml_b200_flash_attn_forward_tokens(const ppml_b200_flash_cfg* cfg, int Lk, 
 /* ---- OP_OUT_PROD -------------------------------------------------------------------------------
  * Replaces out_prod_cuda (src/backend/CUDAKernels.cpp:201; src/cuda/OutProdKernel.cu:211-260):
  * dst[i0,i1,i2,i3] = sum_k s0[i0,k,i2/(ne2/ne02),i3/(ne3/ne03)] * s1[i1,k,i2,i3]; dims in the graph's
- * order (index 0 innermost).  dst is fully overwritten. */
+ * order (index 0 innermost).  dst is fully overwritten.
+ * A plane's result depends on its operands and on the extents of a plane, not on the number of planes.  A long contraction with a
+ * small result (a weight gradient over the tokens: more than 368 k on the CUDA cores, more than 96 on the tensor cores, and an output
+ * tile for at most half the SMs) is summed in interleaved parts: k in slices of 16 (32), part w of W takes the slices w, w + W, ...,
+ * and the parts are added in order.  On the CUDA cores everything is fp32 then too, and closer to the exact sum than one chain.
+ * ppml_b200_out_prod_ordered runs on the CUDA cores and adds k one by one, ascending, at any size: the reference's order, which
+ * out_prod_cuda keeps by default. */
 int ppml_b200_out_prod(const float* src0, const float* src1, float* dst,
                        int64_t ne00, int64_t ne01, int64_t ne02, int64_t ne03,
                        int64_t ne10, int64_t ne11, int64_t ne12, int64_t ne13,
                        int64_t ne0, int64_t ne1, int64_t ne2, int64_t ne3, int path, void* stream);
+int ppml_b200_out_prod_ordered(const float* src0, const float* src1, float* dst,
+                               int64_t ne00, int64_t ne01, int64_t ne02, int64_t ne03,
+                               int64_t ne10, int64_t ne11, int64_t ne12, int64_t ne13,
+                               int64_t ne0, int64_t ne1, int64_t ne2, int64_t ne3, void* stream);
 
 /* ---- OP_TRI_MUL ---------------------------------------------------------------------------------
  * Replaces tri_mul_cuda (src/backend/CUDAKernels.cpp:316; src/cuda/PairKernels.cu:47-77, :514-523).

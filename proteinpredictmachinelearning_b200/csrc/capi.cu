@@ -361,10 +361,10 @@ int ppml_b200_flash_attn_forward(const ppml_b200_flash_cfg* cfg, const float* Q,
                                            O, LSE, path, stream);
 }
 
-int ppml_b200_out_prod(const float* src0, const float* src1, float* dst,
-                       int64_t ne00, int64_t ne01, int64_t ne02, int64_t ne03,
-                       int64_t ne10, int64_t ne11, int64_t ne12, int64_t ne13,
-                       int64_t ne0, int64_t ne1, int64_t ne2, int64_t ne3, int path, void* stream) {
+static int out_prod_any(const float* src0, const float* src1, float* dst,
+                        int64_t ne00, int64_t ne01, int64_t ne02, int64_t ne03,
+                        int64_t ne10, int64_t ne11, int64_t ne12, int64_t ne13,
+                        int64_t ne0, int64_t ne1, int64_t ne2, int64_t ne3, int path, bool ordered, void* stream) {
     if (!src0 || !src1 || !dst || !path_ok(path)) return ST_BAD_ARGS;
     if (ne00 <= 0 || ne01 <= 0 || ne02 <= 0 || ne03 <= 0 || ne10 <= 0 || ne12 <= 0 || ne13 <= 0) return ST_BAD_ARGS;
     if (ne11 != ne01 || ne0 != ne00 || ne1 != ne10 || ne2 < ne02 || ne3 < ne03 || ne2 != ne12 || ne3 != ne13) return ST_BAD_ARGS;
@@ -393,8 +393,22 @@ int ppml_b200_out_prod(const float* src0, const float* src1, float* dst,
     p.a_s2 = ne00 * ne01; p.a_s3 = ne00 * ne01 * ne02; p.a_div2 = ne2 / ne02; p.a_div3 = ne3 / ne03;
     p.b_s2 = ne10 * ne11; p.b_s3 = ne10 * ne11 * ne12;
     p.c_s2 = ne0 * ne1; p.c_s3 = ne0 * ne1 * ne2;
-    p.alpha = 1.0f;
+    p.alpha = 1.0f; p.in_parts = ordered ? 0 : 1;
     return launch_simt_contract(src0, src1, dst, p, 0, as_stream(stream));
+}
+
+int ppml_b200_out_prod(const float* src0, const float* src1, float* dst,
+                       int64_t ne00, int64_t ne01, int64_t ne02, int64_t ne03,
+                       int64_t ne10, int64_t ne11, int64_t ne12, int64_t ne13,
+                       int64_t ne0, int64_t ne1, int64_t ne2, int64_t ne3, int path, void* stream) {
+    return out_prod_any(src0, src1, dst, ne00, ne01, ne02, ne03, ne10, ne11, ne12, ne13, ne0, ne1, ne2, ne3, path, false, stream);
+}
+
+int ppml_b200_out_prod_ordered(const float* src0, const float* src1, float* dst,
+                               int64_t ne00, int64_t ne01, int64_t ne02, int64_t ne03,
+                               int64_t ne10, int64_t ne11, int64_t ne12, int64_t ne13,
+                               int64_t ne0, int64_t ne1, int64_t ne2, int64_t ne3, void* stream) {
+    return out_prod_any(src0, src1, dst, ne00, ne01, ne02, ne03, ne10, ne11, ne12, ne13, ne0, ne1, ne2, ne3, PPML_B200_PATH_SIMT, true, stream);
 }
 
 static int tri_mul_any(const void* left, const void* right, float* dst, int64_t D, int64_t I, int64_t J,

@@ -19,6 +19,7 @@ struct SimtContract {
     long long a_s2, a_s3, a_div2, a_div3;
     long long b_s2, b_s3, c_s2, c_s3;
     long long b_div2, b_div3;   // 0 = 1
+    int in_parts;               // 1: the order of the sum is free (plain products, alpha 1): long contractions are summed in parts
     int vec_c;                  // set by the launcher: 16-byte stores are legal
     const float* bias;
     int bias_seed;              // 1: accumulator starts at bias[n] (fp32 mul_mat); 0: added at the end

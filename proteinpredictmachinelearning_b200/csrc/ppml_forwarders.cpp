@@ -8,7 +8,7 @@
 // Arithmetic of the fp32 entries.  In the reference mul_mat_cuda, out_prod_cuda, tri_mul_cuda and
 // outer_prod_mean_cuda and flash_attn_forward_cuda are exact-fp32 CUDA-core kernels; tf32 tensor cores are opt-in through PPML_MUL_MAT_TC, and
 // only for nodes without a bias (src/backend/CUDAKernels.cpp:822-842).  The forwarders keep that default: with
-// nothing set they run this library's CUDA-core kernels (fp32 accumulation in the reference's order).  The tensor
+// nothing set they run this library's CUDA-core kernels (fp32 accumulation in the reference's order: k ascending).  The tensor
 // cores are switched on by the reference's own variable or by this library's:
 //   PPML_MUL_MAT_TC=<not 0>   tf32 tensor cores for every fp32 entry (attention included: tf32 products, fp32
 //                             softmax), bias included (the epilogue adds it in fp32)
@@ -140,8 +140,10 @@ void out_prod_cuda(const float* src0, const float* src1, float* dst,
                    int64_t ne00, int64_t ne01, int64_t ne02, int64_t ne03,
                    int64_t ne10, int64_t ne11, int64_t ne12, int64_t ne13,
                    int64_t ne0, int64_t ne1, int64_t ne2, int64_t ne3) {
-    const int rc = ppml_b200_out_prod(src0, src1, dst, ne00, ne01, ne02, ne03, ne10, ne11, ne12, ne13, ne0, ne1, ne2, ne3,
-                                      batched_path(), nullptr);
+    const int path = batched_path();
+    const int rc = path == PPML_B200_PATH_SIMT
+                       ? ppml_b200_out_prod_ordered(src0, src1, dst, ne00, ne01, ne02, ne03, ne10, ne11, ne12, ne13, ne0, ne1, ne2, ne3, nullptr)
+                       : ppml_b200_out_prod(src0, src1, dst, ne00, ne01, ne02, ne03, ne10, ne11, ne12, ne13, ne0, ne1, ne2, ne3, path, nullptr);
     if (rc != 0) std::fprintf(stderr, "[ppml_b200] out_prod_cuda failed rc=%d\n", rc);
 }
 

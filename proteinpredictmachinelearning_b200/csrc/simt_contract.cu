@@ -4,15 +4,19 @@
 //   D[p][m][n] = epi( sum_k A[pa][m][k] * B[pb][n][k] )
 //
 // Each output element is one chain of fused multiply-adds with k ascending, the reference's order, so fp32 results agree with
-// its CPU kernels to rounding and do not depend on which of the kernels below, or how many planes, a call runs.
+// its CPU kernels to rounding and do not depend on which of the kernels below, or how many planes, a call runs.  Only out_prod may be
+// asked for without that order, and then sums long contractions in parts (in_parts, below).
 #include "kernels.h"
 
+#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
 #include <type_traits>
 
 #include "common.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace ppml_b200 {
 
@@ -74,6 +78,10 @@ struct Loader {
             ptr[g] += step;
         }
     }
+    __device__ __forceinline__ void skip(long long elems) {
+#pragma unroll
+        for (int g = 0; g < kGroups; ++g) ptr[g] += elems;
+    }
     __device__ __forceinline__ void store(int tid, float* stage) const {
 #pragma unroll
         for (int g = 0; g < kGroups; ++g) {
@@ -109,6 +117,7 @@ struct Loader<T, Fetch::ANY, ROWS, NT> {
         for (int i = 0; i < kElems; ++i) v[i] = (r0 + i * dr < rows_left && k0 + i * dk < k_left) ? to_f32<T>(ptr[i * delta]) : 0.0f;
         ptr += step;
     }
+    __device__ __forceinline__ void skip(long long elems) { ptr += elems; }
     __device__ __forceinline__ void store(int, float* stage) const {
 #pragma unroll
         for (int i = 0; i < kElems; ++i) {
@@ -321,9 +330,7 @@ simt_contract_kernel(const T* __restrict__ A, const T* __restrict__ B, float* __
 // FMAs); with several, shared-memory reads (24 bytes per thread and k: 12 cycles per k and CTA, broadcast or not).  128 x 256 over
 // 2601 tokens 135 -> 24 us, 256 x 256 over 65536 4793 -> 553, 64 x 64 over 65536 3214 -> 526 (64 x 64 tiles of 256 threads before).
 // 2 x 2 outputs per thread on four warps with slices of 32: 28 us and 640; one warp with a 16 x 16 tile: 26 and 613.
-// Dealing the slices to the groups of a cluster and adding the partial sums took 16 and 273 us and came closer to the 64-bit result
-// (1.9e-7 against 9.1e-7 at 2601 tokens), but it is not the order that the callers of this path are promised, and the sum
-// depended on the number of planes.
+// The contraction in parts (below) takes 16 and 273 us for the first two.
 constexpr int kNarrowSlice = 64, kNarrowDepth = 4, kNarrowM = 32, kNarrowN = 16, kNarrowThreads = 64;
 
 __device__ __forceinline__ void cp_async(uint32_t dst, const float* src, bool in, std::integral_constant<int, 16>) {
@@ -420,6 +427,170 @@ simt_contract_narrow_kernel(const float* __restrict__ A, const float* __restrict
     }
 }
 
+// A contraction in parts, for out_prod with a long contraction and a small result where the caller does not ask for one chain: part w of W
+// takes the slices of k w, w + W, ..., ascending, and the result is ((part 0 + part 1) + ...) in fp32.  W follows from M, N and K
+// alone, so the bits do not depend on how many planes a call holds.  The shorter chains come closer to the 64-bit result than one
+// (128 x 256 over 2601 tokens: 1.9e-7 against 9.1e-7).  Where the parts run:
+//
+// simt_contract_split_kernel: a CTA is two or four groups of four warps, a cluster up to 16 CTAs, a group takes one part of a 64 x 64 tile,
+// with stages and a barrier of its own.  The partial tiles are left in shared memory and added piece by piece over the cluster (no
+// atomics).
+// Bound: FMA issue with 16 or more tiles; latency of a group's loads below that (one slice in flight per group), which is why
+// the parts are many and short.  256 x 256 over 65536 tokens 4793 -> 273 us (one CTA per 64 x 64 tile before), 64 x 256 over
+// 30000 1490 -> 63 us, 33 x 32 over 30000 1470 -> 73 us.
+template <Fetch F, int kSplitGroups>
+__global__ void __launch_bounds__(kSplitGroups * 128, 4 / kSplitGroups)
+simt_contract_split_kernel(const float* __restrict__ A, const float* __restrict__ B, float* __restrict__ C, const SimtContract p, int n_tiles) {
+    constexpr int BM = 64, BN = 64;
+    static_assert(BM * BN == 2 * kSlice * (BM + BN), "a partial tile fills its group's stages");
+    extern __shared__ __align__(16) float dyn[];
+    cg::cluster_group cl = cg::this_cluster();
+    const int splits = static_cast<int>(cl.num_blocks()), rank = static_cast<int>(cl.block_rank());
+    const int grp = threadIdx.x >> 7, gtid = threadIdx.x & 127;
+    float* const As = dyn + grp * (BM * BN);
+    float* const Bs = As + 2 * kSlice * BM;
+    const int warp = gtid >> 5, lane = gtid & 31;
+    const int arow = (warp >> 1) * 32 + lane_m(lane) * 4, bcol = (warp & 1) * 32 + lane_n(lane) * 4;
+    const int mt = blockIdx.x / n_tiles;
+    const long long m0 = static_cast<long long>(mt) * BM, n0 = static_cast<long long>(blockIdx.x - mt * n_tiles) * BN;
+    const PlanePtrs<float> pp = plane_ptrs(A, B, C, p, blockIdx.z / splits);
+
+    const long long ways = static_cast<long long>(splits) * kSplitGroups;
+    const long long kbeg = (rank * kSplitGroups + grp) * static_cast<long long>(kSlice), kstep = ways * kSlice;
+    long long k_left = p.K - kbeg;                       // not positive: a group without a share
+    float acc[8][4];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
+    auto group_sync = [&] { asm volatile("bar.sync %0, 128;" ::"r"(grp + 1) : "memory"); };
+    Loader<float, F, BM, 128> la;
+    Loader<float, F, BN, 128> lb;
+    la.init(pp.a, gtid, m0, p.M, kbeg, p.a_sm, p.a_sk, ways);
+    lb.init(pp.b, gtid, n0, p.N, kbeg, p.b_sn, p.b_sk, ways);
+    la.fetch(gtid, clip_slice(k_left));
+    lb.fetch(gtid, clip_slice(k_left));
+    la.store(gtid, As);
+    lb.store(gtid, Bs);
+    group_sync();
+    int buf = 0;
+    for (; k_left > 0; k_left -= kstep, buf ^= 1) {
+        const bool more = k_left > kstep;
+        if (more) {
+            la.fetch(gtid, clip_slice(k_left - kstep));
+            lb.fetch(gtid, clip_slice(k_left - kstep));
+        }
+        mac_slice<F, BM, BN, 4>(As + buf * (kSlice * BM), Bs + buf * (kSlice * BN), arow, bcol, acc);
+        if (more) {
+            la.store(gtid, As + (buf ^ 1) * (kSlice * BM));
+            lb.store(gtid, Bs + (buf ^ 1) * (kSlice * BN));
+        }
+        group_sync();
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+        *reinterpret_cast<float4*>(As + (arow + (i < 4 ? i : 12 + i)) * BN + bcol) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+    cl.sync();
+    for (int e = rank * (kSplitGroups * 128) + static_cast<int>(threadIdx.x); e < BM * BN / 4; e += splits * (kSplitGroups * 128)) {
+        const int r = e / (BN / 4), c = (e % (BN / 4)) * 4;
+        if (m0 + r >= p.M || n0 + c >= p.N) continue;
+        float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int q = 0; q < splits; ++q) {
+            const float* part = cl.map_shared_rank(dyn, q) + r * BN + c;
+#pragma unroll
+            for (int g = 0; g < kSplitGroups; ++g) {
+                const float4 x = *reinterpret_cast<const float4*>(part + g * (BM * BN));
+                s.x += x.x; s.y += x.y; s.z += x.z; s.w += x.w;
+            }
+        }
+        float* dst = pp.c + (m0 + r) * p.c_sm + (n0 + c);
+        const float o[4] = {s.x, s.y, s.z, s.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) if (n0 + c + j < p.N) dst[j] = o[j];
+    }
+    cl.sync();                                           // nobody leaves while a peer still reads
+}
+
+// The same parts one after the other in one CTA, where the planes bring enough tiles for the SMs: simt_contract_kernel's tiles and
+// pipeline over the slices in the order of the parts, each part added to C by the threads that own its elements.
+template <Fetch F, int TN>
+__global__ void __launch_bounds__(128, TN == 8 || F == Fetch::ANY ? 3 : 4)
+simt_contract_parts_kernel(const float* __restrict__ A, const float* __restrict__ B, float* C, const SimtContract p, int n_tiles, int parts) {
+    constexpr int BM = 64, BN = 16 * TN;
+    __shared__ __align__(16) float smem[2 * kSlice * (BM + BN)];
+    float* const As = smem;
+    float* const Bs = smem + 2 * kSlice * BM;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int arow = (warp >> 1) * 32 + lane_m(lane) * 4, bcol = (warp & 1) * (8 * TN) + lane_n(lane) * 4;
+    const long long mt = blockIdx.x / n_tiles;
+    const long long m0 = mt * BM, n0 = (static_cast<long long>(blockIdx.x) - mt * n_tiles) * BN;
+    const int slices = static_cast<int>((p.K + kSlice - 1) / kSlice);
+
+    for (long long plane = blockIdx.z; plane < p.planes; plane += gridDim.z) {
+        const PlanePtrs<float> pp = plane_ptrs(A, B, C, p, plane);
+        float acc[8][TN];
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int j = 0; j < TN; ++j) acc[i][j] = 0.0f;
+        Loader<float, F, BM, 128> la;
+        Loader<float, F, BN, 128> lb;
+        la.init(pp.a, threadIdx.x, m0, p.M, 0, p.a_sm, p.a_sk, parts);
+        lb.init(pp.b, threadIdx.x, n0, p.N, 0, p.b_sn, p.b_sk, parts);
+        // fetches slice s and moves on to the next one of its part, or to the first of the next part
+        auto fetch = [&](int s) {
+            const int k_left = clip_slice(p.K - static_cast<long long>(s) * kSlice);
+            la.fetch(threadIdx.x, k_left);
+            lb.fetch(threadIdx.x, k_left);
+            if (s + parts < slices) return s + parts;
+            const int next = s % parts + 1;
+            la.skip(static_cast<long long>(next - s - parts) * kSlice * p.a_sk);
+            lb.skip(static_cast<long long>(next - s - parts) * kSlice * p.b_sk);
+            return next;
+        };
+        int s = 0, ahead = fetch(0);
+        la.store(threadIdx.x, As);
+        lb.store(threadIdx.x, Bs);
+        __syncthreads();
+        for (int it = 0, buf = 0; it < slices; ++it, buf ^= 1) {
+            const bool more = it + 1 < slices;
+            const int now = s;
+            if (more) { s = ahead; ahead = fetch(s); }
+            mac_slice<F, BM, BN, TN>(As + buf * (kSlice * BM), Bs + buf * (kSlice * BN), arow, bcol, acc);
+            if (now + parts >= slices) {                  // the last slice of its part
+                const bool first = now % parts == 0;
+#pragma unroll
+                for (int jg = 0; jg < TN / 4; ++jg) {
+                    const long long n = n0 + bcol + 32 * jg;
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const long long m = m0 + arow + (i < 4 ? i : 12 + i);
+                        float* c = pp.c + m * p.c_sm + n;
+                        float v[4] = {0.f, 0.f, 0.f, 0.f};
+                        if (m < p.M && n < p.N) {
+                            if (p.vec_c) {
+                                if (!first) *reinterpret_cast<float4*>(v) = load4(c);
+                                *reinterpret_cast<float4*>(c) = make_float4(v[0] + acc[i][4 * jg], v[1] + acc[i][4 * jg + 1], v[2] + acc[i][4 * jg + 2], v[3] + acc[i][4 * jg + 3]);
+                            } else {
+#pragma unroll
+                                for (int j = 0; j < 4; ++j)
+                                    if (n + j < p.N) c[j] = (first ? 0.0f : c[j]) + acc[i][4 * jg + j];
+                            }
+                        }
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) acc[i][4 * jg + j] = 0.0f;
+                    }
+                }
+            }
+            if (more) {
+                la.store(threadIdx.x, As + (buf ^ 1) * (kSlice * BM));
+                lb.store(threadIdx.x, Bs + (buf ^ 1) * (kSlice * BN));
+            }
+            __syncthreads();
+        }
+    }
+}
+
 template <typename T, Fetch F, int WM, int WN, int TN, bool FUSED>
 int launch_tile(const T* A, const T* B, float* C, const SimtContract& p, cudaStream_t st) {
     constexpr int BM = WM * 32, BN = WN * 8 * TN;
@@ -428,6 +599,91 @@ int launch_tile(const T* A, const T* B, float* C, const SimtContract& p, cudaStr
     const unsigned planes = static_cast<unsigned>(p.planes < 32768 ? p.planes : 32768);
     simt_contract_kernel<T, F, WM, WN, TN, FUSED><<<dim3(static_cast<unsigned>(mt * nt), 1, planes), WM * WN * 32, 0, st>>>(A, B, C, p, static_cast<int>(nt));
     return cudaGetLastError() == cudaSuccess ? ST_OK : ST_LAUNCH;
+}
+
+// ---- the contraction in parts
+// Clusters of each size that a B200 holds at once for two and for four groups (cudaOccupancyMaxActiveClusters, 148 SMs); constants, so that
+// the number of parts follows from the extents alone.
+constexpr int kSplitSms = 148;
+constexpr int kResident2[17] = {0, 296, 148, 93, 71, 56, 45, 37, 33, 30, 26, 21, 21, 17, 14, 14, 14};
+constexpr int kResident4[17] = {0, 148, 74, 45, 33, 26, 22, 15, 15, 15, 11, 7, 7, 7, 7, 7, 7};
+
+// Groups per CTA and CTAs per cluster: clusters beyond what the GPU holds at once wait for a second wave, so the size is the one with
+// the fewest slices one after the other for one plane, at three (four from 64 slices on) or more slices per part (with one, many planes
+// waited for the sums: 32 of 128 x 128 over 408 45 us against 19 in one chain; 128 x 128 over 408 itself 7.6 us with three, 8.7 with four).  groups = 1, one chain: a result with a tile for more than half the SMs, or K
+// below 24 slices, where the narrow form is faster (128 x 256 over 225 4.2 us against 5.8, over 408 6.0 and 9.1) and a chain is about as
+// far from the 64-bit result as the forward product's.
+struct SplitPlan { int groups, splits; long long rounds; };
+inline long long split_waves(const int (&resident)[17], int splits, long long tiles) { return (tiles + resident[splits] - 1) / resident[splits]; }
+inline void plan_split(SplitPlan& best, int groups, const int (&resident)[17], long long tiles, long long slices) {
+    const long long least = slices < 64 ? 3 : 4;
+    for (int s = 1; s <= 16 && least * s * groups <= slices; ++s) {
+        const long long rounds = split_waves(resident, s, tiles) * ((slices + s * groups - 1) / (s * groups));
+        if (rounds < best.rounds) best = {groups, s, rounds};
+    }
+}
+SplitPlan plan_parts(const SimtContract& p) {
+    const long long slices = (p.K + kSlice - 1) / kSlice;
+    SplitPlan plan{1, 1, slices};
+    if (!p.in_parts || slices < 24 || p.K > 0x7fffffffLL || p.M > 64LL * kSplitSms || p.N > 64LL * kSplitSms) return plan;
+    const long long tiles = ((p.M + 63) / 64) * ((p.N + 63) / 64);
+    if (2 * tiles > kSplitSms) return plan;
+    plan_split(plan, 2, kResident2, tiles, slices);
+    plan_split(plan, 4, kResident4, tiles, slices);
+    return plan;
+}
+
+template <Fetch F, int G>
+int launch_split(const float* A, const float* B, float* C, const SimtContract& p, int splits, cudaStream_t st) {
+    constexpr int kSmem = G * 64 * 64 * static_cast<int>(sizeof(float));
+    auto kern = simt_contract_split_kernel<F, G>;
+    static bool configured[64] = {false};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) { cudaGetLastError(); return ST_LAUNCH; }
+    if (!configured[dev]) {
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) != cudaSuccess ||
+            cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+            cudaGetLastError();
+            return ST_LAUNCH;
+        }
+        configured[dev] = true;
+    }
+    const int nt = static_cast<int>((p.N + 63) / 64);
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute at{};
+    cfg.gridDim = dim3(static_cast<unsigned>((p.M + 63) / 64 * nt), 1, static_cast<unsigned>(p.planes * splits));
+    cfg.blockDim = dim3(G * 128); cfg.dynamicSmemBytes = kSmem; cfg.stream = st;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = 1; at.val.clusterDim.y = 1; at.val.clusterDim.z = static_cast<unsigned>(splits);
+    cfg.attrs = &at; cfg.numAttrs = 1;
+    if (cudaLaunchKernelEx(&cfg, kern, A, B, C, p, nt) != cudaSuccess) { cudaGetLastError(); return ST_LAUNCH; }
+    return ST_OK;
+}
+
+template <Fetch F, int TN>
+int launch_parts(const float* A, const float* B, float* C, const SimtContract& p, int parts, cudaStream_t st) {
+    const int mt = static_cast<int>((p.M + 63) / 64), nt = static_cast<int>((p.N + 16 * TN - 1) / (16 * TN));
+    const unsigned planes = static_cast<unsigned>(p.planes < 32768 ? p.planes : 32768);
+    simt_contract_parts_kernel<F, TN><<<dim3(static_cast<unsigned>(mt * nt), 1, planes), 128, 0, st>>>(A, B, C, p, nt, parts);
+    return cudaGetLastError() == cudaSuccess ? ST_OK : ST_LAUNCH;
+}
+
+template <Fetch F>
+int launch_in_parts(const float* A, const float* B, float* C, const SimtContract& p, const SplitPlan& plan, cudaStream_t st) {
+    // times (ns): waves of clusters, each 1700 a slice of its groups, 120 a part for the sum and 2000 beside; or CTAs with all parts of
+    // their tiles, 600 a slice and 1600 for adding a part (64 x 64 over 2601 tokens in 54 parts: 64 planes 152 us on clusters, 187 in one
+    // CTA each; in 40 parts 80 on clusters)
+    const long long sms = num_sms(), slices = (p.K + kSlice - 1) / kSlice;
+    const int parts = plan.groups * plan.splits;
+    const long long tiles = ((p.M + 63) / 64) * ((p.N + 63) / 64) * p.planes;
+    const long long wave = 2000 + 120 * parts + 1700 * ((slices + parts - 1) / parts), serial = 600 * slices + 1600 * parts;
+    const long long waves = split_waves(plan.groups == 2 ? kResident2 : kResident4, plan.splits, tiles);
+    if (p.planes <= 16384 / plan.splits && waves * wave <= ((tiles + 2 * sms - 1) / (2 * sms)) * serial)
+        return plan.groups == 2 ? launch_split<F, 2>(A, B, C, p, plan.splits, st) : launch_split<F, 4>(A, B, C, p, plan.splits, st);
+    if constexpr (F != Fetch::ANY) {                      // tiles as for one chain, below
+        if (p.N > 64 && ((p.M + 63) / 64) * ((p.N + 127) / 128) * p.planes >= 3 * sms) return launch_parts<F, 8>(A, B, C, p, parts, st);
+    }
+    return launch_parts<F, 4>(A, B, C, p, parts, st);
 }
 
 // at most half the SMs would have a 64 x 64 tile (so no extent of the launch below is large).  A CTA per SM takes 102 us for the 2601
@@ -468,8 +724,11 @@ int launch_typed(const T* A, const T* B, float* C, const SimtContract& p, cudaSt
                          (p.ne2 == 1 || (p.a_s2 % 4 == 0 && p.b_s2 % 4 == 0)) &&
                          (p.planes == p.ne2 || (p.a_s3 % 4 == 0 && p.b_s3 % 4 == 0));
     if constexpr (std::is_same_v<T, float>) {
+        const bool vec = base_ok && p.a_sm == 1 && p.b_sn == 1 && p.M % 4 == 0 && p.N % 4 == 0 && p.a_sk % 4 == 0 && p.b_sk % 4 == 0;
+        const SplitPlan plan = plan_parts(p);
+        if (plan.groups > 1)
+            return vec ? launch_in_parts<Fetch::VEC_ROW>(A, B, C, p, plan, st) : launch_in_parts<Fetch::ANY>(A, B, C, p, plan, st);
         if (takes_narrow(p)) {
-            const bool vec = base_ok && p.M % 4 == 0 && p.N % 4 == 0 && p.a_sk % 4 == 0 && p.b_sk % 4 == 0;
             return vec ? launch_narrow<4>(A, B, C, p, st) : launch_narrow<1>(A, B, C, p, st);
         }
     }
@@ -499,6 +758,7 @@ int launch_simt_contract(const void* A, const void* B, float* C, const SimtContr
         const void* t = A; A = B; B = t;
     }
     const bool c_al = (reinterpret_cast<uintptr_t>(C) & 15u) == 0 && p.N % 4 == 0 && (p.ne2 == 1 || p.c_s2 % 4 == 0) && (p.planes == p.ne2 || p.c_s3 % 4 == 0);
+    p.in_parts = p.in_parts && p.c_sn == 1 && p.alpha == 1.0f && p.bias == nullptr && !p.clamp && p.opm_L == 0;
     p.vec_c = p.opm_L > 0 ? (c_al && p.opm_B == 1 && p.opm_L % 4 == 0) : (c_al && p.c_sn == 1 && p.c_sm % 4 == 0);
     if (elem == 0) return launch_typed<float>(static_cast<const float*>(A), static_cast<const float*>(B), C, p, st);
     if (elem == 1) return launch_typed<__half>(static_cast<const __half*>(A), static_cast<const __half*>(B), C, p, st);

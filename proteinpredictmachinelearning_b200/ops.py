@@ -268,15 +268,17 @@ def flash_attn_backward_cuda(Q, K, V, O, dO, LSE, bias=None, scale=0.0, causal=F
     return out
 
 
-def out_prod_cuda(s0, s1, path=PATH_AUTO):
-    """s0 [ne03,ne02,K,ne00], s1 [ne13,ne12,K,ne10] (torch order = reversed graph dims) -> [ne3,ne2,ne10,ne00]."""
+def out_prod_cuda(s0, s1, path=PATH_AUTO, ordered=False):
+    """s0 [ne03,ne02,K,ne00], s1 [ne13,ne12,K,ne10] (torch order = reversed graph dims) -> [ne3,ne2,ne10,ne00].  ordered: exact fp32,
+    one ascending chain over K per output (what out_prod_cuda in the library runs by default); path is not used then."""
     s0, s1 = _f32c(s0), _f32c(s1)
     ne03, ne02, ne01, ne00 = s0.shape
     ne13, ne12, ne11, ne10 = s1.shape
     ne2, ne3 = max(ne02, ne12), max(ne03, ne13)
     dst = torch.empty((ne3, ne2, ne10, ne00), device=s0.device, dtype=torch.float32)
-    rc = _lib.load().ppml_b200_out_prod(_p(s0), _p(s1), _p(dst), ne00, ne01, ne02, ne03, ne10, ne11, ne12, ne13,
-                                        ne00, ne10, ne2, ne3, path, _stream())
+    args = (_p(s0), _p(s1), _p(dst), ne00, ne01, ne02, ne03, ne10, ne11, ne12, ne13, ne00, ne10, ne2, ne3)
+    lib = _lib.load()
+    rc = lib.ppml_b200_out_prod_ordered(*args, _stream()) if ordered else lib.ppml_b200_out_prod(*args, path, _stream())
     _check(rc, "out_prod")
     return dst
 

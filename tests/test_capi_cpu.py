@@ -50,6 +50,7 @@ def test_bad_arguments_are_rejected_on_the_host(lib):
     assert lib.ppml_b200_flash_attn_forward(None, p, p, p, None, p, None, 0, None) == 1
     assert lib.ppml_b200_tri_mul(p, p, p, 0, 1, 1, 1, 1, 1.0, 1, 0, None) == 1
     assert lib.ppml_b200_out_prod(p, p, p, 4, 3, 1, 1, 5, 2, 1, 1, 4, 5, 1, 1, 0, None) == 1             # K mismatch
+    assert lib.ppml_b200_out_prod_ordered(p, p, p, 4, 3, 1, 1, 5, 2, 1, 1, 4, 5, 1, 1, None) == 1
     assert lib.ppml_b200_quantize_rows_q8_1(p, p, 33, None) == 1
     assert lib.ppml_b200_q8_0r_bytes(64) == 68
     # entries without a counterpart in the reference follow the same conventions

@@ -936,7 +936,7 @@ def test_exact_contraction_tile_edges(oracle, M, K, N):
 @pytest.mark.parametrize("sa,sb,sc", [(1, 0, 0), (0, 1, 0), (0, 0, 1)])
 def test_exact_contraction_bases_off_16_bytes(M, K, N, sa, sb, sc):
     """Extents in whole groups of four with one base 4 bytes off: element-wise loads, or stores, by the address alone; the bits do not
-    change.  Last case: out_prod over 256 tokens (narrow tiles) as well."""
+    change.  Last case: out_prod over 256 tokens as well, in one chain and in parts."""
     g = torch.Generator(device="cuda").manual_seed(37)
     a, b, c = (torch.zeros(m * n + 1, device="cuda") for m, n in ((M, K), (N, K), (M, N)))
     a[sa:sa + M * K] = torch.randn(M * K, device="cuda", generator=g)
@@ -948,21 +948,56 @@ def test_exact_contraction_bases_off_16_bytes(M, K, N, sa, sb, sc):
     if M == K:
         at = a[sa:sa + M * K].view(1, 1, K, M)                                  # read as [K][M], [K][N]
         bt = b[sb:sb + N * K].view(1, 1, K, N)
-        assert torch.equal(ops.out_prod_cuda(at, bt, path=PATH_SIMT), ops.out_prod_cuda(at.clone(), bt.clone(), path=PATH_SIMT))
+        for ordered in (True, False):
+            assert torch.equal(ops.out_prod_cuda(at, bt, path=PATH_SIMT, ordered=ordered), ops.out_prod_cuda(at.clone(), bt.clone(), path=PATH_SIMT, ordered=ordered))
 
 
 @pytest.mark.parametrize("n0,n1,K,p2,ne02", [(256, 128, 2601, 1, 1), (33, 32, 4099, 1, 1), (36, 132, 65, 2, 1), (8, 4, 64, 1, 1),
                                              (130, 66, 1000, 3, 3), (64, 64, 16 * 64 + 1, 1, 1), (512, 160, 100, 1, 1), (31, 17, 256, 40, 1)])
 def test_exact_contraction_small_result(oracle, n0, n1, K, p2, ne02):
-    """Few output tiles and a long contraction (narrow tiles): one ascending chain per output, bit for bit -- the same as the product of
-    the transposed operands through mul_mat and as each plane by itself -- with rows that are and are not whole groups of four."""
+    """Few output tiles and a long contraction.  Ordered (narrow tiles): one ascending chain per output, bit for bit -- the same as the
+    product of the transposed operands through mul_mat and as each plane by itself.  In parts: a plane gives the bits it has alone.
+    With rows that are and are not whole groups of four."""
     s0, s1 = cases.out_prod_case(n0, n1, K, p2, 1, ne02=ne02, seed=32)
-    got = ops.out_prod_cuda(dev(s0), dev(s1), path=PATH_SIMT)
-    assert cases.rel_err(host(got), oracle.out_prod(s0, s1)) <= TOL_FP32
-    for i in {0, p2 - 1}:
-        t0, t1 = dev(s0[:, i * ne02 // p2]), dev(s1[:, i])                 # [1, K, n0], [1, K, n1]
-        assert torch.equal(got[0, i], ops.mul_mat_cuda(t1[0].t().contiguous(), t0[0].t().contiguous(), path=PATH_SIMT))
-        assert torch.equal(got[0, i], ops.out_prod_cuda(t0[None], t1[None], path=PATH_SIMT)[0, 0])
+    ref = oracle.out_prod(s0, s1)
+    for ordered in (True, False):
+        got = ops.out_prod_cuda(dev(s0), dev(s1), path=PATH_SIMT, ordered=ordered)
+        assert cases.rel_err(host(got), ref) <= TOL_FP32
+        for i in {0, p2 - 1}:
+            t0, t1 = dev(s0[:, i * ne02 // p2]), dev(s1[:, i])             # [1, K, n0], [1, K, n1]
+            assert torch.equal(got[0, i], ops.out_prod_cuda(t0[None], t1[None], path=PATH_SIMT, ordered=ordered)[0, 0])
+            if ordered:
+                assert torch.equal(got[0, i], ops.mul_mat_cuda(t1[0].t().contiguous(), t0[0].t().contiguous(), path=PATH_SIMT))
+
+
+def test_out_prod_cuda_by_its_own_name_keeps_the_order(monkeypatch):
+    """The drop-in launcher with nothing set: one ascending chain over a long contraction."""
+    import ctypes as C
+    from proteinpredictmachinelearning_b200 import _lib
+    for name in ("PPML_B200_MATH", "PPML_MUL_MAT_TC"):
+        monkeypatch.delenv(name, raising=False)
+    fn = _lib.load()["_ZN4ppml13out_prod_cudaEPKfS1_Pfllllllllllll"]
+    fn.restype, fn.argtypes = None, [C.c_void_p] * 3 + [C.c_int64] * 12
+    s0, s1 = (dev(x) for x in cases.out_prod_case(132, 64, 2601, 1, 1, seed=39))
+    got = torch.empty((1, 1, 64, 132), device="cuda")
+    torch.cuda.synchronize()
+    fn(s0.data_ptr(), s1.data_ptr(), got.data_ptr(), 132, 2601, 1, 1, 64, 2601, 1, 1, 132, 64, 1, 1)
+    torch.cuda.synchronize()
+    assert torch.equal(got, ops.out_prod_cuda(s0, s1, ordered=True))
+    assert not torch.equal(got, ops.out_prod_cuda(s0, s1, path=PATH_SIMT))
+
+
+@pytest.mark.parametrize("n0,n1,K,P", [(256, 256, 2601, 40), (64, 64, 700, 200), (33, 31, 300, 300), (128, 160, 97, 160), (100, 70, 1000, 64), (20, 132, 65, 500)])
+def test_exact_out_prod_bits_do_not_depend_on_the_planes(n0, n1, K, P):
+    """The parts of a contraction on a cluster (one plane, a few) and in one CTA (many), with every tile and loader."""
+    g = torch.Generator(device="cuda").manual_seed(38)
+    s0, s1 = (torch.randn((1, P, K, n), device="cuda", generator=g) for n in (n0, n1))
+    whole = ops.out_prod_cuda(s0, s1, path=PATH_SIMT)
+    ref = s1[0].double().transpose(1, 2) @ s0[0].double()
+    assert float((whole[0] - ref).abs().max() / ref.abs().max()) <= TOL_FP32
+    for lo, n in ((0, 1), (P - 1, 1), (1, 3), (0, P // 2)):
+        part = ops.out_prod_cuda(s0[:, lo:lo + n].contiguous(), s1[:, lo:lo + n].contiguous(), path=PATH_SIMT)
+        assert torch.equal(part, whole[:, lo:lo + n]), (lo, n)
 
 
 def test_exact_contraction_is_one_ascending_chain():
@@ -972,7 +1007,7 @@ def test_exact_contraction_is_one_ascending_chain():
     acc = np.zeros((20, 36), np.float32)
     for k in range(700):
         acc = (acc.astype(np.longdouble) + s1[0, 0, k].astype(np.longdouble)[:, None] * s0[0, 0, k].astype(np.longdouble)[None]).astype(np.float32)
-    assert np.array_equal(host(ops.out_prod_cuda(dev(s0), dev(s1), path=PATH_SIMT))[0, 0], acc)
+    assert np.array_equal(host(ops.out_prod_cuda(dev(s0), dev(s1), ordered=True))[0, 0], acc)
     assert np.array_equal(host(ops.mul_mat_cuda(dev(s1[0, 0].T), dev(s0[0, 0].T), path=PATH_SIMT)), acc)
 
 
