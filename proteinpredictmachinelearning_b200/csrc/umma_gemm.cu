@@ -149,7 +149,7 @@ long long parts_ns(const UmmaGemmArgs& a, int BN, int parts, int k_steps) {
 // Parts of the contraction, from M, N and K alone: the cluster size that is fastest for one result, at least two K steps per part (with
 // one, a CTA that computes all parts waits for its sums: 512 planes of 256 x 256 over 408 tokens 107 us in 13 parts, 88 undivided).
 // 1: more than half the SMs have a tile of the general kernel, or there are fewer than four K steps (256 x 256 over 256 tokens,
-// eight of them: 11.7 -> 5.4 us; over 128: 9.4 -> 4.7).
+// eight of them: 11.7 -> 5.4 us; over 128: 9.4 -> 5.2).
 int gemm_parts(const UmmaGemmArgs& a, int general_bn, int k_steps) {
     const long long tiles = static_cast<long long>((a.M + 127) / 128) * ((a.N + general_bn - 1) / general_bn);
     if (!a.may_split || k_steps < 4 || 2 * tiles > kSplitSms) return 1;
