@@ -9,16 +9,16 @@
 //   attn_bwd_dq_kernel   one CTA = 64 query rows of one (batch, head); walks the key tiles of 64; writes dQ and dbias
 //   attn_bwd_dkv_kernel  one CTA = 64 key rows of one (batch, head); walks the query tiles of 64; writes dK and dV
 // Per tile: scores and dP as register tiles over the channels, exp and dS in registers, dS (and P, one after the other through
-// the same buffer) to shared memory as [partner][own row], then the result's register tile over the partners (attn_tile.cuh).  A causal row takes
-// nothing from the partner rows beyond its diagonal, whatever values they hold.
+// the same buffer) to shared memory as [partner][own row], then the result's register tile over the partners (attn_tile.cuh).  A
+// causal row takes nothing from the partner rows beyond its diagonal, whatever values they hold.
 //
 // Bound: instruction issue (fp32 FMAs are half of it: 3 products in one kernel, 4 in the other; FMA pipe 45 % busy at two CTAs
-// per SM).  64 x 8 x 256 x 32 with dbias 1535 -> 510 us (30 TFLOP/s over the seven products), head dim 8 613 -> 259 us, against
+// per SM).  64 x 8 x 256 x 32 with dbias 1535 -> 498 us (30 TFLOP/s over the seven products), head dim 8 613 -> 251 us, against
 // 32-row tiles with a warp per 8 rows, whose lanes read one scalar from shared memory per FMA or two.  The next tile and this
 // tile's bias are requested before the products (255 registers, two CTAs per SM): 573 us with three CTAs per SM that wait for
 // them.  Sequences that fit one tile of 32 rows keep that form (attn_backward_short.cu, with both sides' times); above, the
-// 64-row tiles are faster throughout, also where they are emptiest (256 x 8, 33 rows: 120 -> 76, 343 -> 142 and 641 -> 255 us for
-// head dims 8, 32 and 64; 72 rows: 279 -> 257, 801 -> 510, 1434 -> 916).
+// 64-row tiles are faster throughout, also where they are emptiest (256 x 8, 33 rows: 120 -> 74, 343 -> 138 and 641 -> 251 us for
+// head dims 8, 32 and 64; 72 rows: 279 -> 249, 801 -> 495, 1434 -> 903).
 // Layouts as the forward: Q, K, V, O, dO, dQ, dK, dV [B, h, L, d]; bias [B, h, L, L] with a batch stride (0: shared);
 // dbias [B, h, L, L]; LSE [B, h, L].  d <= 64.
 #include <cuda_runtime.h>
@@ -100,7 +100,7 @@ __device__ __forceinline__ void put4(float* row, int c, int L, bool vec, const f
 // ---- dQ and dbias -------------------------------------------------------------------------------------------------------
 template <int DP> constexpr int dq_smem_floats() { return 5 * DP * kT + kT * kT + 2 * kT; }
 
-template <int DP>
+template <int DP, bool CAUSAL>
 __global__ void __launch_bounds__(kAttnThreads, 2) attn_bwd_dq_kernel(const BwdParams p) {
     extern __shared__ __align__(16) float sm[];
     float* Qt = sm;                                   // own rows, transposed
@@ -142,12 +142,12 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_bwd_dq_kernel(const BwdP
 #pragma unroll
         for (int c = 0; c < AttnOut<DP>::kCols; ++c) o[i][c] = 0.0f;
 
-    const int jend = p.causal ? min(p.L, i0 + kT) : p.L;         // keys past the last row's diagonal are masked for all
+    const int jend = CAUSAL ? min(p.L, i0 + kT) : p.L;           // keys past the last row's diagonal are masked for all
     for (int j0 = 0; j0 < jend; j0 += kT) {
         __syncthreads();                               // the tiles of the previous step are no longer read
         rk.template store<true, true>(Kt, Kr);
         rv.template store<true, false>(Vt, nullptr);
-        const bool diag = p.causal && j0 == i0, fin = !diag || rk.finite();
+        const bool diag = CAUSAL && j0 == i0, fin = !diag || rk.finite();
         const int j = j0 + bcol;
         float4 bi[8];                                  // this tile's bias and the next tile's keys travel during the products
 #pragma unroll
@@ -170,7 +170,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_bwd_dq_kernel(const BwdP
             const int rl = arow + (r < 4 ? r : 12 + r), i = i0 + rl;
             const float lse = Ls[rl], Di = Dr[rl];
             const float bj[4] = {bi[r].x, bi[r].y, bi[r].z, bi[r].w};
-            const int keys = (lse > -CUDART_INF_F ? (p.causal ? min(i + 1, p.L) : p.L) : 0) - j;      // visible ones from column j on
+            const int keys = (lse > -CUDART_INF_F ? (CAUSAL ? min(i + 1, p.L) : p.L) : 0) - j;      // visible ones from column j on
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 s[r][u] = u < keys ? expf(s[r][u] * p.scale + bj[u] - lse) * (dp[r][u] - Di) : 0.0f;
@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_bwd_dq_kernel(const BwdP
         }
     }
     // keys past jend of a causal CTA: dbias stays 0 there
-    if (dbias && p.causal) {
+    if (dbias && CAUSAL) {
         const int j1 = ((jend + kT - 1) / kT) * kT;    // the walked tiles wrote up to here
         for (int r = warp; r < kT; r += 4)
             if (i0 + r < p.L) for (int j = j1 + lane; j < p.L; j += 32) dbias[static_cast<size_t>(i0 + r) * p.L + j] = 0.0f;
@@ -201,7 +201,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_bwd_dq_kernel(const BwdP
 // ---- dK and dV ----------------------------------------------------------------------------------------------------------
 template <int DP> constexpr int dkv_smem_floats() { return 6 * DP * kT + kT * kT + 2 * kT; }
 
-template <int DP>
+template <int DP, bool CAUSAL>
 __global__ void __launch_bounds__(kAttnThreads, 2) attn_bwd_dkv_kernel(const BwdParams p) {
     extern __shared__ __align__(16) float sm[];
     float* Kt = sm;                                   // own rows, transposed
@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_bwd_dkv_kernel(const Bwd
     const size_t base = static_cast<size_t>(bh) * p.L * p.d;
     const float* bias = p.bias ? p.bias + static_cast<size_t>(b) * p.bias_batch_stride + static_cast<size_t>(hh) * p.L * p.L : nullptr;
 
-    const int ibeg = p.causal ? j0 : 0;                // query rows before the first key of the tile see none of it
+    const int ibeg = CAUSAL ? j0 : 0;                  // query rows before the first key of the tile see none of it
     AttnRows<DP> rq, rg, ro;                           // the next query tile on its way: Q, dO, O and the LSE
     float rl;
     auto fetch_queries = [&](int i0) {
@@ -253,7 +253,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_bwd_dkv_kernel(const Bwd
         rg.template store<true, true>(dOt, dOr);
         store_row_dots<DP>(rg, ro, Dr);
         if (threadIdx.x < kT) Ls[threadIdx.x] = rl;
-        const bool diag = p.causal && i0 == j0, fin = !diag || (rq.finite() && rg.finite());
+        const bool diag = CAUSAL && i0 == j0, fin = !diag || (rq.finite() && rg.finite());
         float4 bi[4][2];                               // this tile's bias and the next query tile travel during the products
 #pragma unroll
         for (int u = 0; u < 4; ++u)
@@ -275,7 +275,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_bwd_dkv_kernel(const Bwd
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
             const int i = i0 + bcol + u;
-            keys[u] = (lse[u] > -CUDART_INF_F ? (p.causal ? min(i + 1, p.L) : p.L) : 0) - (j0 + arow);
+            keys[u] = (lse[u] > -CUDART_INF_F ? (CAUSAL ? min(i + 1, p.L) : p.L) : 0) - (j0 + arow);
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const float bj[4] = {bi[u][h].x, bi[u][h].y, bi[u][h].z, bi[u][h].w};
@@ -315,31 +315,35 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_bwd_dkv_kernel(const Bwd
     }
 }
 
-template <int DP>
-int launch_dp(const BwdParams& p, cudaStream_t st) {
+template <int DP, bool CAUSAL>
+int launch_causal(const BwdParams& p, cudaStream_t st) {
     const dim3 grid((p.L + kT - 1) / kT, p.B * p.H);
     constexpr int dq_bytes = dq_smem_floats<DP>() * 4, dkv_bytes = dkv_smem_floats<DP>() * 4;
     static bool configured[64] = {false};
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) { cudaGetLastError(); return ST_LAUNCH; }
     if (!configured[dev]) {
-        if (cudaFuncSetAttribute(attn_bwd_dq_kernel<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, dq_bytes) != cudaSuccess ||
-            cudaFuncSetAttribute(attn_bwd_dkv_kernel<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, dkv_bytes) != cudaSuccess) {
+        if (cudaFuncSetAttribute(attn_bwd_dq_kernel<DP, CAUSAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, dq_bytes) != cudaSuccess ||
+            cudaFuncSetAttribute(attn_bwd_dkv_kernel<DP, CAUSAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, dkv_bytes) != cudaSuccess) {
             cudaGetLastError();
             return ST_LAUNCH;
         }
         configured[dev] = true;
     }
     if (p.dQ || p.dbias) {
-        attn_bwd_dq_kernel<DP><<<grid, kAttnThreads, dq_bytes, st>>>(p);
+        attn_bwd_dq_kernel<DP, CAUSAL><<<grid, kAttnThreads, dq_bytes, st>>>(p);
         if (cudaGetLastError() != cudaSuccess) return ST_LAUNCH;
     }
     if (p.dK || p.dV) {
-        attn_bwd_dkv_kernel<DP><<<grid, kAttnThreads, dkv_bytes, st>>>(p);
+        attn_bwd_dkv_kernel<DP, CAUSAL><<<grid, kAttnThreads, dkv_bytes, st>>>(p);
         if (cudaGetLastError() != cudaSuccess) return ST_LAUNCH;
     }
     return ST_OK;
 }
+
+// causal calls have instances of their own: what their tiles ask for cost the others 3 % (515 against 498 us at 64 x 8 x 256 x 32)
+template <int DP>
+int launch_dp(const BwdParams& p, cudaStream_t st) { return p.causal ? launch_causal<DP, true>(p, st) : launch_causal<DP, false>(p, st); }
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 

@@ -6,7 +6,7 @@
 // Arithmetic contract as attn_rowwarp_kernel: denominator l + eps, LSE = m + log(l + eps), a row without a visible key (or, with
 // ft > 0, whose first ft scores are all -inf) gives O = 0, LSE = -inf.
 //
-// Bound: instruction issue, about half of it the FMAs of the two products.  64 x 8 x 256 x 32 with a shared bias 497 -> 199 us, 51 x 8 x
+// Bound: instruction issue, about half of it the FMAs of the two products.  256 x 8 x 256 x 32 with a shared bias 2375 -> 749 us, 51 x 8 x
 // 51 x 32 32 -> 16 us back to back in a graph (33 -> 19 as calls) against attn_rowwarp_kernel (16 rows per CTA, one key per lane: a
 // scalar shared-memory read and a shuffle for every few FMAs).
 #include <cuda_runtime.h>
@@ -29,7 +29,7 @@ struct ExactAttn {
 
 template <int DP> constexpr int exact_smem_floats() { return 3 * DP * kAttnTile + kAttnTile * kAttnTile + kAttnTile; }
 
-template <typename T, int DP>
+template <typename T, int DP, bool CAUSAL>
 __global__ void __launch_bounds__(kAttnThreads, DP == 32 ? 3 : 2)
 attn_exact_kernel(const T* __restrict__ Q, const T* __restrict__ K, const T* __restrict__ V, const float* __restrict__ bias,
                   float* __restrict__ O, float* __restrict__ LSE, const ExactAttn p) {
@@ -47,7 +47,7 @@ attn_exact_kernel(const T* __restrict__ Q, const T* __restrict__ K, const T* __r
     const T* Kb = K + b * lay.k_b + hh * lay.k_h;
     const T* Vb = V + b * lay.v_b + hh * lay.v_h;
     const float* bh = bias ? bias + static_cast<size_t>(b) * p.bias_batch_stride + static_cast<size_t>(hh) * p.L * static_cast<size_t>(p.Lk) : nullptr;
-    const int jend = p.causal ? min(min(i0 + kT, p.L), p.Lk) : p.Lk;          // keys needed by any row of this CTA
+    const int jend = CAUSAL ? min(min(i0 + kT, p.L), p.Lk) : p.Lk;            // keys needed by any row of this CTA
 
     AttnRows<DP> rk, rv;                              // the next key tile on its way
     {
@@ -72,7 +72,7 @@ attn_exact_kernel(const T* __restrict__ Q, const T* __restrict__ K, const T* __r
         __syncthreads();                              // the tiles of the previous step are no longer read
         rk.template store<true, false>(Kt, nullptr);
         rv.template store<false, true>(nullptr, Vr);
-        const bool diag = p.causal && j0 == i0, fin = !diag || rv.finite();
+        const bool diag = CAUSAL && j0 == i0, fin = !diag || rv.finite();
         if (j0 + kT < jend) {
             rk.fetch(Kb, lay.k_l, j0 + kT, p.Lk, p.d, p.vec_k);
             rv.fetch(Vb, lay.v_l, j0 + kT, p.Lk, p.d, p.vec_v);
@@ -86,7 +86,7 @@ attn_exact_kernel(const T* __restrict__ Q, const T* __restrict__ K, const T* __r
 #pragma unroll
         for (int r = 0; r < 8; ++r) {
             const int i = i0 + arow + (r < 4 ? r : 4 + r);
-            const int keys = (i < p.L ? (p.causal ? min(i + 1, p.Lk) : p.Lk) : 0) - j;       // visible ones from column j on
+            const int keys = (i < p.L ? (CAUSAL ? min(i + 1, p.Lk) : p.Lk) : 0) - j;       // visible ones from column j on
             float bj[4] = {0.f, 0.f, 0.f, 0.f};
             if (bh && keys > 0) {
                 const float* br = bh + static_cast<size_t>(i) * p.Lk + j;
@@ -185,21 +185,26 @@ attn_exact_kernel(const T* __restrict__ Q, const T* __restrict__ K, const T* __r
     }
 }
 
-template <typename T, int DP>
-int launch_typed(const T* Q, const T* K, const T* V, const float* bias, float* O, float* LSE, int B, const ExactAttn& p, cudaStream_t st) {
+template <typename T, int DP, bool CAUSAL>
+int launch_causal(const T* Q, const T* K, const T* V, const float* bias, float* O, float* LSE, int B, const ExactAttn& p, cudaStream_t st) {
     constexpr int bytes = exact_smem_floats<DP>() * 4;
     static bool configured[64] = {false};
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) { cudaGetLastError(); return ST_LAUNCH; }
     if (!configured[dev]) {
-        if (cudaFuncSetAttribute(attn_exact_kernel<T, DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) {
+        if (cudaFuncSetAttribute(attn_exact_kernel<T, DP, CAUSAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) {
             cudaGetLastError();
             return ST_LAUNCH;
         }
         configured[dev] = true;
     }
-    attn_exact_kernel<T, DP><<<dim3((p.L + kAttnTile - 1) / kAttnTile, p.H, B), kAttnThreads, bytes, st>>>(Q, K, V, bias, O, LSE, p);
+    attn_exact_kernel<T, DP, CAUSAL><<<dim3((p.L + kAttnTile - 1) / kAttnTile, p.H, B), kAttnThreads, bytes, st>>>(Q, K, V, bias, O, LSE, p);
     return cudaGetLastError() == cudaSuccess ? ST_OK : ST_LAUNCH;
+}
+
+template <typename T, int DP>
+int launch_typed(const T* Q, const T* K, const T* V, const float* bias, float* O, float* LSE, int B, const ExactAttn& p, cudaStream_t st) {
+    return p.causal ? launch_causal<T, DP, true>(Q, K, V, bias, O, LSE, B, p, st) : launch_causal<T, DP, false>(Q, K, V, bias, O, LSE, B, p, st);
 }
 
 // rows that start on 4-element boundaries: base and every stride

@@ -611,8 +611,8 @@ constexpr int kResident4[17] = {0, 148, 74, 45, 33, 26, 22, 15, 15, 15, 11, 7, 7
 // Groups per CTA and CTAs per cluster: clusters beyond what the GPU holds at once wait for a second wave, so the size is the one with
 // the fewest slices one after the other for one plane, at three (four from 64 slices on) or more slices per part (with one, many planes
 // waited for the sums: 32 of 128 x 128 over 408 45 us against 19 in one chain; 128 x 128 over 408 itself 7.6 us with three, 8.7 with four).  groups = 1, one chain: a result with a tile for more than half the SMs, or K
-// below 24 slices, where the narrow form is faster (128 x 256 over 225 4.2 us against 5.8, over 408 6.0 and 9.1) and a chain is about as
-// far from the 64-bit result as the forward product's.
+// below 24 slices, where the narrow form is faster (128 x 256 over 225 4.3 us against 5.8) and a chain is about as far from the 64-bit
+// result as the forward product's; above, the chain falls behind in its error first (408: 6.0 us, in parts 7.7), then in time (1000 k).
 struct SplitPlan { int groups, splits; long long rounds; };
 inline long long split_waves(const int (&resident)[17], int splits, long long tiles) { return (tiles + resident[splits] - 1) / resident[splits]; }
 inline void plan_split(SplitPlan& best, int groups, const int (&resident)[17], long long tiles, long long slices) {
